@@ -303,8 +303,9 @@ int wema_cuda_server_stats(wema_cuda_server *srv, int reset, wema_cuda_serve_sta
  *   - the temporal filter's step at 2, 4 and 8 coefficient positions per
  *     thread (a 2^23-position trial plane) and keeps the fastest (4, the
  *     default, unless another is more than 3% faster);
- *   - the batched guided filter's sweep at 64, 128 and 256 output rows per
- *     segment (a 3840x8640 trial frame) and keeps the fastest (64 until then);
+ *   - the batched guided filter's sweep with its rows split evenly over the
+ *     warps (the setting 64, the default) and at 128 and 256 output rows per
+ *     segment (a 3840x8640 trial frame) and keeps the fastest;
  *   - the batched luma DWT level-0 kernels, forward and inverse, in nine
  *     variants each: CTAs per SM asked of the register allocator {1 (the
  *     compiler's choice), 3, 4} x lines lifted per warp at a time {2, 4, 8}

@@ -59,6 +59,7 @@ struct Launch {
     unsigned total = 0;
     size_t params_off = 0, map_off = 0;   // device offsets in the tick's table
     bool any16 = false;                   // some task has FP16 planes (planes_fp16)
+    int mode = -2;                        // guided transfer: the tasks' row form, -1 when they differ, -2 none
     void reset(size_t e) {
         elem = e;
         params.clear();
@@ -67,6 +68,7 @@ struct Launch {
         nblk.clear();
         total = 0;
         any16 = false;
+        mode = -2;
     }
     void add(const void* p, unsigned x, unsigned y, unsigned blocks) {
         if (blocks == 0) return;
@@ -616,7 +618,12 @@ public:
                 tp.h16 = S.cfg.planes_fp16;
                 unsigned gx, gy;
                 const unsigned b = transfer_grid(tp, gx, gy);
-                LK[tp.edge_aware ? L_XFER_GUIDED : L_XFER_GAUSS].add(&tp, gx, gy, b);
+                Launch& lx = LK[tp.edge_aware ? L_XFER_GUIDED : L_XFER_GAUSS];
+                lx.add(&tp, gx, gy, b);
+                if (tp.edge_aware) {
+                    const int mode = transfer_rows_mode(tp);
+                    lx.mode = lx.mode == -2 || lx.mode == mode ? mode : -1;
+                }
             }
         }
         // ---- the table image, its buffer, one H2D copy
@@ -704,8 +711,8 @@ public:
                    go(g, L_INV0_COLOR, [&] { return launch_dwt_inv_multi(3, kOutRgb, (const InvLevelParams*)P(g, L_INV0_COLOR), M(g, L_INV0_COLOR), L[g][L_INV0_COLOR].total, L[g][L_INV0_COLOR].any16, st); }, "inverse DWT");
         };
         auto xfer = [&](int g, cudaStream_t st) {
-            return go(g, L_XFER_GUIDED, [&] { return launch_transfer_multi(1, (const TransferParams*)P(g, L_XFER_GUIDED), M(g, L_XFER_GUIDED), L[g][L_XFER_GUIDED].total, st); }, "luma transfer") &&
-                   go(g, L_XFER_GAUSS, [&] { return launch_transfer_multi(0, (const TransferParams*)P(g, L_XFER_GAUSS), M(g, L_XFER_GAUSS), L[g][L_XFER_GAUSS].total, st); }, "luma transfer");
+            return go(g, L_XFER_GUIDED, [&] { return launch_transfer_multi(1, (const TransferParams*)P(g, L_XFER_GUIDED), M(g, L_XFER_GUIDED), L[g][L_XFER_GUIDED].total, L[g][L_XFER_GUIDED].mode, st); }, "luma transfer") &&
+                   go(g, L_XFER_GAUSS, [&] { return launch_transfer_multi(0, (const TransferParams*)P(g, L_XFER_GAUSS), M(g, L_XFER_GAUSS), L[g][L_XFER_GAUSS].total, 0, st); }, "luma transfer");
         };
         // a stage over every group in turn, between its timing marks
         auto all = [&](auto stage, int tstage, cudaStream_t st) {
@@ -756,13 +763,13 @@ public:
         if (steady) {
             // what the graph holds: the table, every launch's blocks and offsets,
             // the device's kernel variants
-            std::vector<long long> sig = {(long long)(uintptr_t)t.dev, dwt_variant(device, 0), dwt_variant(device, 1), G};
+            std::vector<long long> sig = {(long long)(uintptr_t)t.dev, dwt_variant(device, 0), dwt_variant(device, 1), guided_rows(device), G};
             for (int g = 0; g < G; g++)
                 for (const Launch& l : L[g]) {
                     sig.push_back(l.total);
                     sig.push_back((long long)l.params_off);
                     sig.push_back((long long)l.map_off);
-                    sig.push_back(l.any16);
+                    sig.push_back(l.any16 + 2 * l.mode);
                 }
             if (sig != t.sig) {
                 drop_graphs(t);

@@ -126,7 +126,7 @@ struct TransferParams {
     uint8_t* out_u8;            // output RGB24 (optional)
     float* out_f32;             // output float RGB (optional)
     int edge_aware;             // 1: guided filter r=4 eps=0.01; 0: 5-tap Gaussian
-    int seg_rows;               // guided filter: output rows per sweep segment (0: the device's)
+    int seg_rows;               // guided filter: output rows per unit of work (0: filled in)
     int h16;                    // gray_out is an FP16 plane (planes_fp16)
 };
 cudaError_t launch_transfer(const TransferParams& p, cudaStream_t st);
@@ -184,13 +184,17 @@ cudaError_t iir_autotune(int dev, float ms[3], int* chosen);
 cudaError_t launch_iir_multi(const void* d_args, const int* d_map, unsigned blocks, int preseed,
                              cudaStream_t st);
 unsigned transfer_grid(TransferParams& p, unsigned& gx, unsigned& gy);
-// guided filter rows per sweep segment on a device (default 64)
+// how the guided sweep reads the stream's rows (spatial.cu's kRows...)
+int transfer_rows_mode(const TransferParams& p);
+// rows per sweep segment on a device (64, the default: the work is split evenly
+// over the warps in units of 16 rows)
 int guided_rows(int dev);
 bool guided_set_rows(int dev, int rows);
 // times the sweep at each candidate segment height, keeps the fastest
 cudaError_t guided_autotune(int dev, const int* cand, int nc, float* ms, int* chosen);
+// mode: the guided tasks' common transfer_rows_mode, or -1 when they differ
 cudaError_t launch_transfer_multi(int edge_aware, const TransferParams* d_params, const int* d_map,
-                                  unsigned blocks, cudaStream_t st);
+                                  unsigned blocks, int mode, cudaStream_t st);
 // a tick's parameter table from pinned host memory (its device-mapped
 // address) into device memory, read by a kernel over the host link: no copy
 // engine, so it never queues behind a frame copy; bytes rounded up to 16
