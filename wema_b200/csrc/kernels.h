@@ -139,16 +139,20 @@ cudaError_t launch_passthrough(const TransferParams& p, cudaStream_t st);
 struct WindowParams {
     long long pu;               // unique positions
     int ws, head;               // window size, ring slot of the oldest sample
+    int newest;                 // ring slot of the frame's own sample
     int bilateral;
-    int fp16;                   // ring elements are __half (else float)
-    int h16;                    // the delta plane written is FP16 (planes_fp16)
+    int fp16;                   // ring elements are __half (ring_fp16), else float
+    int h16;                    // coef and delta are FP16 planes (planes_fp16)
+    const float* coef[3];       // per channel: the frame's coefficients (null: pushed already)
+    void* ring[3];
+    float* delta[3];
     float time_w[256];
 };
-// coef: FP16 plane when h16 (planes_fp16); ring: __half elements when fp16 (ring_fp16)
-cudaError_t launch_ring_push(const float* coef, int h16, void* ring, int fp16, long long pu, int slot,
-                             cudaStream_t st);
-cudaError_t launch_window(const WindowParams& wp, const void* ring, float* delta,
-                          cudaStream_t st);
+cudaError_t window_prepare_device();
+// the frame's coefficients into their ring slot (while the ring fills)
+cudaError_t launch_ring_push(const WindowParams& wp, int channels, cudaStream_t st);
+// the same push, and the deltas of the full window
+cudaError_t launch_window(const WindowParams& wp, int channels, cudaStream_t st);
 
 // ---- batched launches: one launch of a kernel over many streams --------------
 // Every launch takes a device array of per-task parameters and a task map

@@ -570,7 +570,10 @@ WEMA_API void temporal_filter_apply(const TemporalFilter* filt, const TemporalBu
     wp.pu = (long long)buf->num_positions;
     wp.ws = buf->window_size;
     wp.head = buf->head;
+    wp.newest = (buf->head + buf->window_size - 1) % buf->window_size;
     wp.bilateral = bilateral;
+    wp.ring[0] = buf->phase_buffer;
+    wp.delta[0] = d_delta;
     const int ws = buf->window_size, center = ws / 2;
     const float ts = (float)ws * 0.15f;
     const float inv2 = 0.5f / (ts * ts);
@@ -578,7 +581,7 @@ WEMA_API void temporal_filter_apply(const TemporalFilter* filt, const TemporalBu
         const float d = (float)(t - center);
         wp.time_w[t] = expf(-(d * d) * inv2);
     }
-    if (!cuda_ok(launch_window(wp, buf->phase_buffer, d_delta, tls.st), "window filter")) return;
+    if (!cuda_ok(launch_window(wp, 1, tls.st), "window filter")) return;
     if (!cuda_ok(cudaMemcpyAsync(delta_phi_filtered, d_delta, buf->num_positions * sizeof(float),
                                  cudaMemcpyDeviceToHost, tls.st),
                  "D2H"))

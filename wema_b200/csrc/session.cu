@@ -53,6 +53,7 @@ bool ensure_device(int dev) {
     if (!cuda_ok(dwt_prepare_device(), "DWT kernel setup")) return false;
     if (!cuda_ok(spatial_prepare_device(), "spatial kernel setup")) return false;
     if (!cuda_ok(thr_prepare_device(), "threshold kernel setup")) return false;
+    if (!cuda_ok(window_prepare_device(), "window kernel setup")) return false;
     ready[dev] = 1;
     return true;
 }
@@ -391,24 +392,27 @@ bool Session::run(const uint8_t* in_u8, const float* in_f32, uint8_t* out_u8, fl
                 return false;
         launches += nch;
     } else {
-        for (int c = 0; c < nch; c++)
-            if (!cuda_ok(launch_ring_push(q.coef[c], cfg.planes_fp16, ring[c], cfg.ring_fp16, pu, head, s_tmp),
-                         "ring push"))
-                return false;
-        launches += nch;
+        WindowParams wp{};
+        wp.newest = head;
         head = (head + 1) % cfg.temporal_window;
         if (filled < cfg.temporal_window) filled++;
         q.passthrough = filled < cfg.temporal_window;   // wema.c:924-929
         q.alpha[0] = cfg.amp_factor;
         q.alpha[1] = q.alpha[2] = cfg.amp_factor * 0.5f;
-        if (!q.passthrough) {
-            WindowParams wp{};
-            wp.pu = pu;
-            wp.ws = cfg.temporal_window;
-            wp.head = head;   // oldest sample (temporal_filter.c:221)
-            wp.bilateral = cfg.bilateral_temp;
-            wp.fp16 = cfg.ring_fp16;
-            wp.h16 = cfg.planes_fp16;
+        wp.pu = pu;
+        wp.ws = cfg.temporal_window;
+        wp.head = head;   // oldest sample (temporal_filter.c:221)
+        wp.bilateral = cfg.bilateral_temp;
+        wp.fp16 = cfg.ring_fp16;
+        wp.h16 = cfg.planes_fp16;
+        for (int c = 0; c < nch; c++) {
+            wp.coef[c] = q.coef[c];
+            wp.ring[c] = ring[c];
+            wp.delta[c] = q.delta[c];
+        }
+        if (q.passthrough) {
+            if (!cuda_ok(launch_ring_push(wp, nch, s_tmp), "ring push")) return false;
+        } else {
             const int ws = cfg.temporal_window, center = ws / 2;
             const float ts = (float)ws * 0.15f;
             const float inv2 = 0.5f / (ts * ts);
@@ -416,11 +420,9 @@ bool Session::run(const uint8_t* in_u8, const float* in_f32, uint8_t* out_u8, fl
                 const float d = (float)(t - center);
                 wp.time_w[t] = expf(-(d * d) * inv2);
             }
-            for (int c = 0; c < nch; c++)
-                if (!cuda_ok(launch_window(wp, ring[c], q.delta[c], s_tmp), "window filter"))
-                    return false;
-            launches += nch;
+            if (!cuda_ok(launch_window(wp, nch, s_tmp), "window filter")) return false;
         }
+        launches++;
     }
     mark(2 * ST_TEMPORAL + 1, s_tmp);
     if (!cuda_ok(cudaEventRecord(q.ev_tmp, s_tmp), "event record")) return false;
