@@ -76,33 +76,13 @@ __device__ __forceinline__ Mono compose(Mono a, Mono b) {   // a first, then b
 __device__ __forceinline__ int apply(int m, Mono d) { return m + ((m & 1) ? d.d1 : d.d0); }
 __device__ __forceinline__ int apply(int m, int2 d) { return m + ((m & 1) ? d.y : d.x); }
 
-// effect of adding |x| (bits ua, sign cleared) to any s of biased exponent eb
-__device__ __forceinline__ Mono elem_mono(uint32_t ua, int eb) {
-    const int ea_raw = (int)(ua >> 23);
-    const int ea = max(ea_raw, 1);
-    const uint32_t ma = (ua & 0x7FFFFFu) | (ea_raw ? 0x800000u : 0u);
-    const int sh = eb - ea;
-    const int shc = min(max(sh, 1), 31);
-    const int q = (int)(ma >> shc);
-    const uint32_t r2 = ma << (32 - shc);          // remainder bits, aligned to the top
-    const int up = r2 > 0x80000000u;
-    const int tie = r2 == 0x80000000u;
-    const int qo = q & 1;
-    Mono m;
-    m.d0 = q + (up | (tie & qo));
-    m.d1 = q + (up | (tie & (qo ^ 1)));
-    if (sh <= 0) m = {SAT, SAT};
-    return m;
-}
-
 __device__ __forceinline__ float from_m(int m, int eb) {
     return __uint_as_float(((uint32_t)eb << 23) | ((uint32_t)m & 0x7FFFFFu));
 }
 
 // Sequential reader of the 6-slot flat array (slots 3-5 mirror 2-0).
 // cur_seek() places it on the (level, slot) segment holding index i;
-// cur_addr() advances segment by segment, so a run of nearby indices costs one
-// division.  levels == 0 views coef as a plain flat array of off6[0] elements.
+// cur_addr() advances segment by segment.  levels == 0 views coef as a plain flat array of off6[0] elements.
 struct Cursor {
     const float* base;           // element at seg0
     long long seg0, seg1;        // current segment [seg0, seg1)
@@ -128,10 +108,9 @@ __device__ __forceinline__ void cur_seek(const PyrView& v, Cursor& c, long long 
     for (int k = 1; k < 4; k++)
         if (k < v.levels && i >= v.off6[k]) l = k;
     c.l = l;
-    const long long r = i - v.off6[l];
-    c.slot = (r < 0x7fffffffLL && v.n[l] < 0x7fffffffLL) ? (int)((int)r / (int)v.n[l])
-                                                           : (int)(r / v.n[l]);
-    if (c.slot > 5) c.slot = 5;
+    // (a frame's 6 n stays below 2^31: sessions are capped at 2^28 pixels)
+    const int r = (int)(i - v.off6[l]), n = (int)v.n[l];
+    c.slot = (r >= n) + (r >= 2 * n) + (r >= 3 * n) + (r >= 4 * n) + (r >= 5 * n);
     cur_set(v, c);
 }
 
@@ -312,10 +291,14 @@ __device__ __forceinline__ void thr_prefix_body(const ThrArgs& a, int bx, int by
 // increments do not depend on parity, a monoid is a plain integer sum and the
 // order of summation is free: thread ln reads float4s 32k + ln (coalesced),
 // which always hold lanes 4(ln & 1) .. 4(ln & 1) + 3, and the sums meet by
-// shuffles.  A warp that meets an exact half takes lane_monoids.
-// Sub-chunks per CTA.  A warp that meets an exact half takes the much slower
-// lane_monoids; small CTAs free their slot as soon as their own warps finish
+// shuffles.  A warp that meets an exact half takes run_monoid.
+// Sub-chunks per CTA.  A warp that meets an exact half takes the slower
+// run_monoid; small CTAs free their slot as soon as their own warps finish
 // instead of holding it for the slowest of eight.
+// (320x240: 39 -> 6.8 us with the halves' path out of registers and shared
+// memory instead of ballots over reloaded elements, and sub-chunks over several
+// segments loaded at once instead of one element after the other; 3840x2160
+// 34 -> 15 us; the 48-stream tick's two launches 211 -> 148 us.)
 constexpr int MON_WARPS = 2;
 // CTAs per SM asked of the register allocator: 10 x 2 warps at 96 registers
 // (8 would allow 128 registers but only 16 warps per SM for a latency-bound kernel)
@@ -354,84 +337,40 @@ __device__ __forceinline__ float scale_of(int eb) {
 }
 constexpr float RND = 8388608.0f;   // 2^23
 
-// Monoids of this thread's four lanes (4 * (ln & 1) + i) over a sub-chunk
-// that contains exact halves (or elements of 2^23 increments and more).  The
-// elements are reloaded through the first-level cache in the warp's float4
-// layout: thread ln holds lane-elements 16k + (ln >> 1), k < 16.  An exact half
-// rounds m + n + 1/2 to the even neighbour, so m is even after it: only a
-// lane's first half depends on the start parity p, and each half adds n plus
-// (parity of m before it) xor (n & 1), where that parity counts the odd
-// increments since the start (p included) or since the previous half.
-// Ballots in lane-element order give those counts.
-__device__ __forceinline__ void lane_monoids(const PyrView& v, long long main, long long i0,
-                                             const float* p, bool vec, bool one, int ln,
-                                             const float (&scale)[4], Mono (&out)[4]) {
-    const int half = ln & 1;
-    const unsigned hmask = half ? 0xAAAAAAAAu : 0x55555555u;
-#pragma unroll 1
-    for (int i = 0; i < 4; i++) {
-        const float sci = i == 0 ? scale[0] : i == 1 ? scale[1] : i == 2 ? scale[2] : scale[3];
-        float S = 0.0f;
-        int cp = 0, first = 1, c1 = 0, cfix = 0;
-        Cursor cl;
-        if (!vec && !one && i0 < main) cur_seek(v, cl, i0);
-#pragma unroll 2
-        for (int k = 0; k < 2 * G / 32; k++) {
-            float x;
-            if (vec) {
-                const float4 x4 = __ldg(reinterpret_cast<const float4*>(p) + 32 * k + ln);
-                x = i == 0 ? x4.x : i == 1 ? x4.y : i == 2 ? x4.z : x4.w;
-            } else {
-                const long long e = 4 * (32 * k + ln) + i;
-                x = one ? __ldg(p + e) : (i0 + e < main ? *cur_addr(v, cl, i0 + e) : 0.0f);
-            }
-            const float q = fabsf(x) * sci;
-            const float r = __fsub_rn(__fadd_rn(q, RND), RND);
-            const bool tie = fabsf(q - r) == 0.5f;
-            const float n = tie ? __fsub_rn(q, 0.5f) : r;
-            S += n;
-            const int nbit = tie ? ((int)n & 1) : 0;
-            const int pbit = tie ? 0 : ((int)fminf(r, 16777216.0f) & 1);
-            const unsigned tm0 = __ballot_sync(FULL, tie) & hmask;
-            const unsigned pm = __ballot_sync(FULL, pbit) & hmask;
-            const unsigned nm = __ballot_sync(FULL, nbit) & hmask;
-            unsigned tm = tm0, done = 0u;
-            while (tm) {
-                const unsigned b = tm & (0u - tm);
-                cp ^= __popc(pm & (b - 1u) & ~done) & 1;
-                const int nb = (nm & b) != 0;
-                if (first) { c1 = cp ^ nb; first = 0; }
-                else cfix += cp ^ nb;
-                cp = 0;
-                done = (b << 1) - 1u;
-                tm &= tm - 1u;
-            }
-            cp ^= __popc(pm & ~done) & 1;
-        }
-#pragma unroll
-        for (int d = 2; d < 32; d <<= 1) S += __shfl_xor_sync(FULL, S, d);
-        const int base = (int)fminf(S, (float)SAT) + cfix;
-        const Mono m = {min(base + (first ? 0 : c1), SAT), min(base + (first ? 0 : (1 ^ c1)), SAT)};
-        if (i == 0) out[0] = m;
-        else if (i == 1) out[1] = m;
-        else if (i == 2) out[2] = m;
-        else out[3] = m;
+// The elements of a warp's sub-chunk in shared memory for run_monoid:
+// lane-element e of lane j at 8 e + j + 8 (e / 64), so that the warp's 32 readers
+// (lane j, quarter q at element 64 q + s) and its float4 writers hit distinct banks
+constexpr int TIE_BUF = 8 * G + 8 * (G / 64);
+
+// One thread's part of the parity monoids of a sub-chunk that contains exact
+// halves (or elements of 2^23 increments and more): lane ln & 7, lane-elements
+// 64 (ln >> 3) .. + 63 in order, for one candidate's scale.  An exact half rounds
+// m + n + 1/2 to the even neighbour, so it adds n plus the parity of m + n.
+// q is cut at 2^23, which leaves the binade from any m (a NaN likewise), and
+// the increment is read from the bits of q + 2^23.
+__device__ __forceinline__ Mono run_monoid(const float* x, float scale) {
+    Mono d = mono_id();
+#pragma unroll 8
+    for (int s = 0; s < G / 4; s++) {
+        const float q = fminf(fabsf(x[8 * s]) * scale, RND);
+        const float t = __fadd_rn(q, RND);
+        const float off = __fsub_rn(q, __fsub_rn(t, RND));
+        const int n = (int)(__float_as_uint(t) - 0x4B000000u) - (off == -0.5f);   // the half's floor
+        const int tie = fabsf(off) == 0.5f;
+        d.d0 += n;
+        d.d1 += n;
+        d.d0 += tie & d.d0;
+        d.d1 += tie & ~d.d1;             // from an odd m
     }
+    return {min(d.d0, SAT), min(d.d1, SAT)};
 }
 
-// The 64 elements of thread ln in the warp's float4 layout when the
-// sub-chunk straddles a (level, slot) segment or is not 16-byte aligned.  Out
-// of line (and reading the view from shared memory) so that the common path
-// stays small in the instruction cache.
-__device__ __noinline__ void load_generic(const PyrView* sv, long long main, long long i0,
-                                          const float* p, bool one, int ln, float* out) {
-    Cursor cu;
-    if (!one && i0 < main) cur_seek(*sv, cu, i0);
-    for (int k = 0; k < 2 * G / 32; k++)
-        for (int i = 0; i < 4; i++) {
-            const long long e = 4 * (32 * k + ln) + i;
-            out[4 * k + i] = one ? __ldg(p + e) : (i0 + e < main ? *cur_addr(*sv, cu, i0 + e) : 0.0f);
-        }
+// the four quarters' monoids composed: lane ln's in thread ln < 8
+__device__ __forceinline__ Mono join_quarters(Mono m) {
+#pragma unroll
+    for (int d = 8; d <= 16; d <<= 1)
+        m = compose(m, Mono{__shfl_down_sync(FULL, m.d0, d), __shfl_down_sync(FULL, m.d1, d)});
+    return m;
 }
 
 __device__ __forceinline__ void thr_monoids_body(const ThrArgs& a, int bx, int by) {
@@ -439,15 +378,11 @@ __device__ __forceinline__ void thr_monoids_body(const ThrArgs& a, int bx, int b
     const PyrView& v = a.v[ch];
     const ThrGeom g = thr_geom(v.off6[v.levels]);
     const ThrScratch& sc = a.s[ch];
-    __shared__ PyrView sv;
-    if (threadIdx.x == 0) {
-        sv = v;
-        if (bx == 0 && a.sub0 == 0) *sc.counter = 0u;   // the walk's lane counter
-    }
-    __syncthreads();
+    __shared__ __align__(16) float tie_buf[MON_WARPS][TIE_BUF];
+    if (threadIdx.x == 0 && bx == 0 && a.sub0 == 0) *sc.counter = 0u;   // the walk's lane counter
     const int warp = threadIdx.x >> 5, ln = threadIdx.x & 31;
     const int sub = a.sub0 + bx * MON_WARPS + warp;
-    if (sub >= g.nsub) return;   // whole warps only; no block barrier follows
+    if (sub >= g.nsub) return;   // whole warps only; there is no block barrier
     const int half = ln & 1;     // this thread's lanes: 4 * half + i
     const long long i0 = (long long)sub * (8 * G);
     Cursor cu;
@@ -465,104 +400,109 @@ __device__ __forceinline__ void thr_monoids_body(const ThrArgs& a, int bx, int b
             xv[k][0] = x.x; xv[k][1] = x.y; xv[k][2] = x.z; xv[k][3] = x.w;
         }
     } else {
-        float tmp[8 * G / 32];
-        load_generic(&sv, g.main, i0, p, one, ln, tmp);
+        // not 16-byte aligned, or over several (level, slot) segments: the elements
+        // one by one, segment after segment (uniform), a segment's loads all in flight
 #pragma unroll
         for (int k = 0; k < 2 * G / 32; k++)
 #pragma unroll
-            for (int i = 0; i < 4; i++) xv[k][i] = tmp[4 * k + i];
+            for (int i = 0; i < 4; i++) xv[k][i] = 0.0f;
+        const long long end = min(i0 + 8 * G, g.main);
+        for (long long at = i0; at < end;) {
+            const long long upto = min(end, cu.seg1);
+            const unsigned lo = (unsigned)(at - i0), cnt = (unsigned)(upto - at);
+            const float* const q = cu.base + (i0 - cu.seg0) + 4 * ln;
+#pragma unroll
+            for (int k = 0; k < 2 * G / 32; k++)
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (4u * (unsigned)(32 * k + ln) + i - lo < cnt) xv[k][i] = __ldg(q + 128 * k + i);
+            at = upto;
+            if (at < end) cur_addr(v, cu, at);
+        }
     }
     int ep, eq;                  // candidates of lane ln & 7
     sub_candidates(a, sc, g, (long long)(ln & 7) * g.nsub, sub, ep, eq);
-    int EP[4], EQ[4];
+    const float scp = scale_of(ep), scq = scale_of(eq);
     float sc4[4], sq4[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        EP[i] = __shfl_sync(FULL, ep, 4 * half + i);
-        EQ[i] = __shfl_sync(FULL, eq, 4 * half + i);
-        sc4[i] = scale_of(EP[i]);
-        sq4[i] = scale_of(EQ[i]);
+        sc4[i] = __shfl_sync(FULL, scp, 4 * half + i);
+        sq4[i] = __shfl_sync(FULL, scq, 4 * half + i);
     }
-    float sp[4], sq[4], ps[4];
+    float sp[4], sq[4];
     float dmax = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 4; i++) { sp[i] = 0.0f; sq[i] = 0.0f; ps[i] = 0.0f; }
+    for (int i = 0; i < 4; i++) { sp[i] = 0.0f; sq[i] = 0.0f; }
+    // five operations per element: q never leaves the fused multiply-adds
 #pragma unroll
     for (int k = 0; k < 2 * G / 32; k++) {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const float a = fabsf(xv[k][i]);
-            const float q = a * sc4[i];
-            const float r = __fsub_rn(__fadd_rn(q, RND), RND);
+            const float r = __fsub_rn(__fmaf_rn(fabsf(xv[k][i]), sc4[i], RND), RND);
             sp[i] += r;
-            dmax = fmaxf(dmax, fabsf(q - r));
-            ps[i] += a;
+            dmax = fmaxf(dmax, fabsf(__fmaf_rn(fabsf(xv[k][i]), sc4[i], -r)));
         }
     }
-    const bool has_q = __any_sync(FULL, (EQ[0] | EQ[1] | EQ[2] | EQ[3]) != 0);
+    const bool has_q = __any_sync(FULL, eq != 0);
     if (has_q) {   // secondary candidates
 #pragma unroll
         for (int k = 0; k < 2 * G / 32; k++) {
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const float q = fabsf(xv[k][i]) * sq4[i];
-                const float r = __fsub_rn(__fadd_rn(q, RND), RND);
+                const float r = __fsub_rn(__fmaf_rn(fabsf(xv[k][i]), sq4[i], RND), RND);
                 sq[i] += r;
-                dmax = fmaxf(dmax, fabsf(q - r));
+                dmax = fmaxf(dmax, fabsf(__fmaf_rn(fabsf(xv[k][i]), sq4[i], -r)));
             }
         }
     }
     // |q - r| reaches 0.5 only at an exact half or at q >= 2^23
-    Mono mp4[4], mq4[4];
-    if (__any_sync(FULL, dmax >= 0.5f)) {
-        lane_monoids(v, g.main, i0, p, vec, one, ln, sc4, mp4);
-        if (has_q) {
-            lane_monoids(v, g.main, i0, p, vec, one, ln, sq4, mq4);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; i++) mq4[i] = mono_id();
-        }
-    } else {
+    const bool ties = __any_sync(FULL, dmax >= 0.5f);
+    Mono MP = mono_id(), MQ = mono_id();   // thread L < 8: lane L's
+    float rs = 0.0f;                       // and its sum of |x|, for the walk's prediction
+    // v[i] (lane 4 (ln & 1) + i) summed over the threads of its lane; thread L < 8
+    // gets lane L's, from thread L >> 2, entry L & 3
+    auto lane_sums = [&](float (&v)[4]) {
+        float mine = 0.0f;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
 #pragma unroll
-            for (int d = 2; d < 32; d <<= 1) {
-                sp[i] += __shfl_xor_sync(FULL, sp[i], d);
-                sq[i] += __shfl_xor_sync(FULL, sq[i], d);
-            }
-            const int a0 = (int)fminf(sp[i], (float)SAT), a1 = (int)fminf(sq[i], (float)SAT);
-            mp4[i] = {a0, a0};
-            mq4[i] = {a1, a1};
+            for (int d = 2; d < 32; d <<= 1) v[i] += __shfl_xor_sync(FULL, v[i], d);
+            const float t = __shfl_sync(FULL, v[i], (ln >> 2) & 1);
+            if ((ln & 3) == i) mine = t;
         }
-    }
-    int EPw[4];   // candidate actually written (0 when it cannot be scaled)
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-#pragma unroll
-        for (int d = 2; d < 32; d <<= 1) ps[i] += __shfl_xor_sync(FULL, ps[i], d);
-        EPw[i] = (EP[i] > 0 && sc4[i] == 0.0f) ? 0 : EP[i];
-    }
-    // thread L < 8 takes lane L from thread L >> 2, entry L & 3
-    const int src = (ln >> 2) & 1, ent = ln & 3;
-    Mono MP = mono_id(), MQ = mono_id();
-    float rs = 0.0f;
-    int epw = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int a0 = __shfl_sync(FULL, mp4[i].d0, src), a1 = __shfl_sync(FULL, mp4[i].d1, src);
-        const int b0 = __shfl_sync(FULL, mq4[i].d0, src), b1 = __shfl_sync(FULL, mq4[i].d1, src);
-        const float a2 = __shfl_sync(FULL, ps[i], src);
-        const int e2 = __shfl_sync(FULL, EPw[i], src);
-        if (ent == i) {
-            MP = {a0, a1};
-            MQ = {b0, b1};
-            rs = a2;
-            epw = e2;
+        return mine;
+    };
+    if (!ties) {   // no parity: both entries alike
+        const float s0 = lane_sums(sp);
+        const int n0 = (int)fminf(s0, (float)SAT);
+        MP = {n0, n0};
+        rs = s0 * __uint_as_float((uint32_t)max(ep - 23, 0) << 23);   // increments of 2^(ep - 150)
+        if (has_q) {
+            const int n1 = (int)fminf(lane_sums(sq), (float)SAT);
+            MQ = {n1, n1};
         }
+    } else {
+        float* const buf = tie_buf[warp];
+#pragma unroll
+        for (int k = 0; k < 2 * G / 32; k++)
+            *reinterpret_cast<float4*>(buf + 128 * k + 4 * ln + 8 * (k >> 2)) =
+                make_float4(xv[k][0], xv[k][1], xv[k][2], xv[k][3]);
+        __syncwarp();
+        const float* x = buf + (8 * (G / 4) + 8) * (ln >> 3) + (ln & 7);
+        MP = join_quarters(run_monoid(x, scp));
+        if (has_q) MQ = join_quarters(run_monoid(x, scq));
+    }
+    if (ties || __any_sync(FULL, scp == 0.0f)) {   // no sum from the increments: the elements' own
+        float ps[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int k = 0; k < 2 * G / 32; k++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) ps[i] += fabsf(xv[k][i]);
+        rs = lane_sums(ps);
     }
     if (ln < 8) {   // lane ln: its own ep / eq
-        ep = epw;
-        if (ep == 0 || scale_of(eq) == 0.0f) eq = 0;
+        if (scp == 0.0f) ep = 0;          // (a candidate that cannot be scaled is dropped)
+        if (ep == 0 || scq == 0.0f) eq = 0;
         const long long row = (long long)ln * g.nsub;
         sc.part[row + sub] = (double)rs;
         sc.candp[row + sub] = make_int4(ep, MP.d0, MP.d1, eq);
