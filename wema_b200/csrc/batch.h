@@ -602,7 +602,7 @@ public:
                 unsigned gx, gy;
                 if (l == 0 && nch == 3) iq.out_u8 = out[k];
                 Launch& li = LK[l == 0 ? (nch == 3 ? L_INV0_COLOR : L_INV0_LUMA) : L_INV1 - (l - 1)];
-                const unsigned b = dwt_inv_grid(iq, l == 0 && nch == 3 ? 1 : nch, gx, gy);
+                const unsigned b = dwt_inv_grid(iq, l == 0 && nch == 3 ? 1 : nch, l == 0 && nch == 3 ? kOutRgb : kOutPlanes, gx, gy);
                 li.add(&iq, gx, gy, b);
                 li.any16 |= iq.h16 != 0;
             }

@@ -26,6 +26,7 @@
 // inward by at most two lanes, all inside the halo.  Arithmetic is the
 // reference's: x = fma(left + right, c, x), scalings as separate multiplies
 // (dwt.c:45-170 as GCC -Ofast evaluates it), so coefficients are bit-exact.
+#include <algorithm>
 #include <atomic>
 #include <type_traits>
 
@@ -33,6 +34,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "multi.cuh"
+#include "sweep.cuh"
 
 namespace wema {
 
@@ -572,6 +574,149 @@ __device__ __forceinline__ void dwt_inv_body(const InvLevelParams& p, int bx, in
     }
 }
 
+constexpr int INV_Q = 2;
+constexpr int SW_RES = 5;                // sweep CTAs resident per SM
+// ---- inverse sweep (sweep.cuh): one channel, planes out.  Per pair of rows a
+// lane takes Q neighbouring elements of LL and of the three bands with their
+// deltas (16-byte loads, issued a pair of rows ahead), amplifies, lifts down the
+// columns and across the two finished rows, and writes 2 Q neighbouring samples
+// of each.
+// what a sweep of one channel uses of its level
+struct InvSweep {
+    int ow, oh, sw, sh, n, unit;
+    const float *ll, *coef, *delta;
+    float* out;
+    float thr, al;
+    bool out16, vec, ovec;
+    __device__ __forceinline__ InvSweep(const InvLevelParams& g, int z, bool h16)
+        : ow(g.ow), oh(g.oh), sw(g.sw), sh(g.sh), n((int)g.n), unit(g.unit) {
+        ll = z == 0 ? g.ll[0] : z == 1 ? g.ll[1] : g.ll[2];
+        coef = z == 0 ? g.coef[0] : z == 1 ? g.coef[1] : g.coef[2];
+        delta = z == 0 ? g.delta[0] : z == 1 ? g.delta[1] : g.delta[2];
+        out = z == 0 ? g.out_planes[0] : z == 1 ? g.out_planes[1] : g.out_planes[2];
+        al = z == 0 ? g.alpha[0] : z == 1 ? g.alpha[1] : g.alpha[2];
+        thr = g.thr[z];
+        out16 = h16 && g.out16;
+        // every row of every plane starts at a vector
+        const uintptr_t in = reinterpret_cast<uintptr_t>(coef) | reinterpret_cast<uintptr_t>(delta);
+        vec = !(sw & (INV_Q - 1)) && !(reinterpret_cast<uintptr_t>(ll) & (4 * INV_Q - 1)) &&
+              !(in & (h16 ? 2 * INV_Q - 1 : 4 * INV_Q - 1));
+        ovec = !out16 && !(ow & 3) && !(reinterpret_cast<uintptr_t>(out) & 15);
+    }
+};
+
+template <int Q, bool H16>
+struct InvRows {
+    float ll[Q], x[3][Q], d[3][Q];       // LH, HH, HL and their deltas
+
+    // the elements of a plane's Q neighbours from element i; vec: aligned, all there
+    static __device__ __forceinline__ void take(const float* p, int i, bool h, bool vec, int n, float (&v)[Q]) {
+        if (vec) {
+            if (h) {
+                const __half* q = reinterpret_cast<const __half*>(p) + i;
+#pragma unroll
+                for (int k = 0; k < Q; k += 2) {
+                    const float2 w = __half22float2(__ldg(reinterpret_cast<const __half2*>(q + k)));
+                    v[k] = w.x; v[k + 1] = w.y;
+                }
+            } else if constexpr (Q == 2) {
+                const float2 w = __ldg(reinterpret_cast<const float2*>(p + i));
+                v[0] = w.x; v[1] = w.y;
+            } else {
+                const float4 w = __ldg(reinterpret_cast<const float4*>(p + i));
+                v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < Q; k++)
+                if (k < n) v[k] = pl_ld(p, i + k, h);
+        }
+    }
+    // row pair j; g: the lane's first pair
+    __device__ __forceinline__ void issue(const InvSweep& p, int j, int g) {
+        const int n = p.sw - g;
+        if (n <= 0) return;
+        const int ie = (mirror(2 * j, p.oh) >> 1) * p.sw + g, io = (mirror(2 * j + 1, p.oh) >> 1) * p.sw + g;
+        const int N = p.n;
+        take(p.ll, ie, false, p.vec, n, ll);
+        take(p.coef, io, H16, p.vec, n, x[0]);
+        take(p.coef, N + io, H16, p.vec, n, x[1]);
+        take(p.coef, 2 * N + ie, H16, p.vec, n, x[2]);
+        take(p.delta, io, H16, p.vec, n, d[0]);
+        take(p.delta, N + io, H16, p.vec, n, d[1]);
+        take(p.delta, 2 * N + ie, H16, p.vec, n, d[2]);
+    }
+};
+
+template <int Q, bool H16, bool EDGE>
+__device__ __forceinline__ void inv_sweep(const InvSweep& p, const Strip<Q>& s, int ya, int yb) {
+    const int lane = threadIdx.x & 31;
+    const int g = s.p0 + Q * lane;
+    const int ow = p.ow, oh = p.oh;
+    const bool live = !EDGE || oh >= 2;
+    const bool writer = Q * lane >= s.lo && Q * lane < s.hi;
+    const float thr = p.thr, al = p.al;
+    float* const out = p.out;
+
+    ColumnInverse<Q> L, H;
+#pragma unroll
+    for (int k = 0; k < Q; k++) {
+        L.o0[k] = L.e1[k] = L.o1[k] = L.e2[k] = 0.0f;
+        H.o0[k] = H.e1[k] = H.o1[k] = H.e2[k] = 0.0f;
+    }
+    InvRows<Q, H16> r;
+    const int j1 = yb + 2;
+    r.issue(p, ya - 2, g);
+#pragma unroll 1
+    for (int j = ya - 2; j < j1; j++) {
+        float e[Q], o[Q], he[Q], ho[Q];
+#pragma unroll
+        for (int k = 0; k < Q; k++) {
+            e[k] = r.ll[k];
+            o[k] = fabsf(r.x[0][k]) > thr ? __fmaf_rn(r.d[0][k], al, r.x[0][k]) : r.x[0][k];
+            ho[k] = fabsf(r.x[1][k]) > thr ? __fmaf_rn(r.d[1][k], al, r.x[1][k]) : r.x[1][k];
+            he[k] = fabsf(r.x[2][k]) > thr ? __fmaf_rn(r.d[2][k], al, r.x[2][k]) : r.x[2][k];
+        }
+        if (j + 1 < j1) r.issue(p, j + 1, g);   // in flight while this pair of rows is lifted
+        L.step(e, o, live);
+        H.step(he, ho, live);
+        const int y = j - 2;
+        if (y < ya) continue;
+        row_inverse<Q, EDGE>(e, he, g, ow);
+        row_inverse<Q, EDGE>(o, ho, g, ow);
+        if (!writer) continue;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if (2 * y + h >= oh) break;
+            const float (&a)[Q] = h ? o : e;
+            const float (&b)[Q] = h ? ho : he;
+            const int at = (2 * y + h) * ow + 2 * g;
+            if (p.ovec && 2 * (g + Q) <= ow) {
+#pragma unroll
+                for (int k = 0; k < Q; k += 2)
+                    *reinterpret_cast<float4*>(out + at + 2 * k) = make_float4(a[k], b[k], a[k + 1], b[k + 1]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < Q; k++) {
+                    if (2 * (g + k) < ow) pl_st(out, at + 2 * k, a[k], p.out16);
+                    if (2 * (g + k) + 1 < ow) pl_st(out, at + 2 * k + 1, b[k], p.out16);
+                }
+            }
+        }
+    }
+}
+
+// units u0 .. u0 + n - 1 (p.unit pairs of rows each) of a CTA's group of strips
+template <int Q, bool H16>
+__device__ __forceinline__ void inv_segment(const InvSweep& p, int group, int u0, int n) {
+    const Strip<Q> s(group * SW_WARPS + (threadIdx.x >> 5), p.sw);
+    if (s.hi <= s.lo) return;
+    const int ya = u0 * p.unit, yb = min(ya + n * p.unit, p.sh);
+    const bool edge = (p.ow % (2 * Q) != 0 && s.p0 + 32 * Q >= p.sw) || p.ow < 2 || p.oh < 2;
+    if (edge) inv_sweep<Q, H16, true>(p, s, ya, yb);
+    else inv_sweep<Q, H16, false>(p, s, ya, yb);
+}
+
 // ------------------------------------------------------------- wrappers
 // one stream per launch, and the batched form (task = stream; params in device
 // memory, one entry per task).  The batched luma kernels also come in tuning
@@ -650,6 +795,31 @@ __global__ void __launch_bounds__(DWT_THREADS, C == 1 ? 4 : 3) k_dwt_inv(InvLeve
         dwt_inv_body<C, OUT, LPW_DEF, false, true>(p, blockIdx.x, blockIdx.y, blockIdx.z);
     else dwt_inv_body<C, OUT, LPW_DEF, H16, false>(p, blockIdx.x, blockIdx.y, blockIdx.z);
 }
+// planes out: a sweep; the channel is the units' third index
+template <bool H16>
+__global__ void __launch_bounds__(SW_THREADS, SW_RES) k_dwt_inv_planes(InvLevelParams pg, int units) {
+    const int per = (pg.sh + pg.unit - 1) / pg.unit;
+    const int strips = (pg.sw + SW_WARPS * SW_LANES * INV_Q - 1) / (SW_WARPS * SW_LANES * INV_Q);
+    int2 u = unit_share(units, blockIdx.x, gridDim.x);
+    while (u.x < u.y) {
+        const int row = u.x % per, col = u.x / per, n = min(u.y - u.x, per - row);
+        inv_segment<INV_Q, H16>(InvSweep(pg, col / strips, H16), col % strips, row, n);
+        u.x += n;
+    }
+}
+template <bool ANY16>
+__global__ void __launch_bounds__(SW_THREADS, SW_RES)
+    k_dwt_inv_planes_multi(const InvLevelParams* __restrict__ ps, const int* __restrict__ map) {
+    int2 u = unit_share(map[1 + map[0]], blockIdx.x, gridDim.x);
+    while (u.x < u.y) {
+        const TaskBlock t = task_block(map, u.x);
+        const InvLevelParams& p = ps[t.task];
+        const int n = min(u.y - u.x, map[map[0] + 2 + t.task] - t.x);
+        if (ANY16 && p.h16) inv_segment<INV_Q, true>(InvSweep(p, t.z, true), t.y, t.x, n);
+        else inv_segment<INV_Q, false>(InvSweep(p, t.z, false), t.y, t.x, n);
+        u.x += n;
+    }
+}
 template <int C, int OUT, int MINB, int LPW, bool ANY16>
 __global__ void __launch_bounds__(DWT_THREADS, MINB)
     k_dwt_inv_multi(const InvLevelParams* __restrict__ ps, const int* __restrict__ map) {
@@ -700,6 +870,8 @@ static size_t fwd_smem(int C) { return (size_t)C * PLANE * sizeof(float); }
 static size_t inv_smem(int C) { return (size_t)C * PLANE * sizeof(float); }
 size_t dwt_smem_bytes(int C) { return fwd_smem(C); }
 
+constexpr int SW_UNIT = 4;               // pairs of rows per unit of a sweep's work
+
 static unsigned tiles_of(int pairs) { return (unsigned)((pairs + TP - 1) / TP); }
 
 template <class K>
@@ -728,10 +900,37 @@ unsigned dwt_fwd_grid(const FwdLevelParams& p, int channels_z, unsigned& gx, uns
     gy = tiles_of(p.sh);
     return gx * gy * (unsigned)channels_z;
 }
-unsigned dwt_inv_grid(const InvLevelParams& p, int channels_z, unsigned& gx, unsigned& gy) {
-    gx = tiles_of((p.ow + 1) / 2);
-    gy = tiles_of((p.oh + 1) / 2);
+unsigned dwt_inv_grid(InvLevelParams& p, int channels_z, int out_mode, unsigned& gx, unsigned& gy) {
+    if (out_mode == kOutPlanes) {        // a sweep: units of rows, strips
+        p.unit = SW_UNIT;
+        gx = (unsigned)((p.sh + p.unit - 1) / p.unit);
+        gy = (unsigned)sweep_groups(p.sw, INV_Q);
+    } else {
+        gx = tiles_of((p.ow + 1) / 2);
+        gy = tiles_of((p.oh + 1) / 2);
+    }
     return gx * gy * (unsigned)channels_z;
+}
+
+// CTAs of a sweep over `units` units of SW_UNIT pairs of rows, an even share each:
+// a segment of m units costs m SW_UNIT + 4 steps (two pairs of rows of
+// halo on either side), a step about 2 + k with k CTAs on the SM (0.5 us alone,
+// 1.5 us with five).
+static int sweep_ctas(int units) {
+    constexpr int kSm = 148;
+    int best = units;
+    long long least = -1;
+    for (int k = 1; k <= SW_RES; k++) {
+        const int most = kSm * k;
+        const int m = std::max(1, (units + most - 1) / most);
+        const int ctas = (units + m - 1) / m;
+        const long long cost = (m * SW_UNIT + 4LL) * (2 + (ctas + kSm - 1) / kSm);
+        if (least < 0 || cost <= least) {
+            least = cost;
+            best = ctas;
+        }
+    }
+    return best;
 }
 
 cudaError_t launch_dwt_fwd_multi(int mode, int channels, const FwdLevelParams* d_params,
@@ -774,20 +973,9 @@ cudaError_t launch_dwt_inv_multi(int channels, int out_mode, const InvLevelParam
         return cudaGetLastError();
     }
     if (out_mode != kOutPlanes) return cudaErrorInvalidValue;
-    const int v = dwt_variant(dwt_dev_now(), 1);
-    const size_t sm = inv_smem(1);
-#define WEMA_INV_CASE(I, MB, LP)                                                                        \
-    case I:                                                                                             \
-        if (any16) k_dwt_inv_multi<1, kOutPlanes, MB, LP, true><<<blocks, DWT_THREADS, sm, st>>>(d_params, d_map); \
-        else k_dwt_inv_multi<1, kOutPlanes, MB, LP, false><<<blocks, DWT_THREADS, sm, st>>>(d_params, d_map); \
-        break;
-    switch (v) {
-        WEMA_INV_CASE(0, 1, 2) WEMA_INV_CASE(1, 1, 4) WEMA_INV_CASE(2, 1, 8)
-        WEMA_INV_CASE(3, 3, 2) WEMA_INV_CASE(4, 3, 4) WEMA_INV_CASE(5, 3, 8)
-        WEMA_INV_CASE(6, 4, 2) WEMA_INV_CASE(7, 4, 4) WEMA_INV_CASE(8, 4, 8)
-        default: return cudaErrorInvalidValue;
-    }
-#undef WEMA_INV_CASE
+    const int ctas = sweep_ctas((int)blocks);
+    if (any16) k_dwt_inv_planes_multi<true><<<ctas, SW_THREADS, 0, st>>>(d_params, d_map);
+    else k_dwt_inv_planes_multi<false><<<ctas, SW_THREADS, 0, st>>>(d_params, d_map);
     return cudaGetLastError();
 }
 
@@ -815,9 +1003,13 @@ cudaError_t launch_dwt_fwd(int mode, int channels, const FwdLevelParams& p, cuda
 
 cudaError_t launch_dwt_inv(int channels, int out_mode, const InvLevelParams& p, cudaStream_t st) {
     const unsigned tx = tiles_of((p.ow + 1) / 2), ty = tiles_of((p.oh + 1) / 2);
-    if (out_mode == kOutPlanes && (channels == 1 || channels == 3))
-        if (p.h16) k_dwt_inv<1, kOutPlanes, true><<<dim3(tx, ty, channels), DWT_THREADS, inv_smem(1), st>>>(p);
-        else k_dwt_inv<1, kOutPlanes, false><<<dim3(tx, ty, channels), DWT_THREADS, inv_smem(1), st>>>(p);
+    if (out_mode == kOutPlanes && (channels == 1 || channels == 3)) {
+        InvLevelParams q = p;
+        unsigned gx, gy;
+        const int units = (int)dwt_inv_grid(q, channels, kOutPlanes, gx, gy);
+        if (p.h16) k_dwt_inv_planes<true><<<sweep_ctas(units), SW_THREADS, 0, st>>>(q, units);
+        else k_dwt_inv_planes<false><<<sweep_ctas(units), SW_THREADS, 0, st>>>(q, units);
+    }
     else if (out_mode == kOutRgb && channels == 3)
         if (p.h16) k_dwt_inv<3, kOutRgb, true><<<dim3(tx, ty, 1), DWT_THREADS, inv_smem(3), st>>>(p);
         else k_dwt_inv<3, kOutRgb, false><<<dim3(tx, ty, 1), DWT_THREADS, inv_smem(3), st>>>(p);
@@ -898,12 +1090,12 @@ cudaError_t dwt_autotune(int dev, float fwd_ms[9], float inv_ms[9], int* fwd_bes
     ip.out_planes[0] = out;
     if ((e = cudaMemcpy(dp, &fp, sizeof fp, cudaMemcpyHostToDevice)) != cudaSuccess) return done(e);
     char* dpi = static_cast<char*>(dp) + sizeof(FwdLevelParams);
-    if ((e = cudaMemcpy(dpi, &ip, sizeof ip, cudaMemcpyHostToDevice)) != cudaSuccess) return done(e);
     unsigned gx, gy;
     const unsigned fblocks = dwt_fwd_grid(fp, 1, gx, gy);
     const int fmap[5] = {1, 0, (int)fblocks, (int)gx, (int)gy};
-    const unsigned iblocks = dwt_inv_grid(ip, 1, gx, gy);
+    const unsigned iblocks = dwt_inv_grid(ip, 1, kOutPlanes, gx, gy);
     const int imap[5] = {1, 0, (int)iblocks, (int)gx, (int)gy};
+    if ((e = cudaMemcpy(dpi, &ip, sizeof ip, cudaMemcpyHostToDevice)) != cudaSuccess) return done(e);
     int* map = static_cast<int*>(dmap);
     for (int inv = 0; inv < 2; inv++) {
         if ((e = cudaMemcpy(map, inv ? imap : fmap, sizeof fmap, cudaMemcpyHostToDevice)) != cudaSuccess)

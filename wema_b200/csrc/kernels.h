@@ -48,6 +48,7 @@ struct InvLevelParams {
     float* out_f32;             // kOutRgb: float RGB output (optional)
     int h16;                    // coef and delta are FP16 planes (ll stays FP32)
     int out16;                  // out_planes are FP16 (the level-0 reconstruction of planes_fp16)
+    int unit;                   // planes out: pairs of rows per unit of work (filled in by the launch)
 };
 
 cudaError_t dwt_prepare_device();
@@ -158,7 +159,7 @@ cudaError_t launch_window(const WindowParams& wp, int channels, cudaStream_t st)
 // Every launch takes a device array of per-task parameters and a task map
 // (multi.cuh); `blocks` is the sum of the tasks' grids.
 unsigned dwt_fwd_grid(const FwdLevelParams& p, int channels_z, unsigned& gx, unsigned& gy);
-unsigned dwt_inv_grid(const InvLevelParams& p, int channels_z, unsigned& gx, unsigned& gy);
+unsigned dwt_inv_grid(InvLevelParams& p, int channels_z, int out_mode, unsigned& gx, unsigned& gy);
 // any16: some task has FP16 planes (planes_fp16); false selects the kernel
 // compiled for FP32 planes only
 cudaError_t launch_dwt_fwd_multi(int mode, int channels, const FwdLevelParams* d_params,

@@ -33,4 +33,9 @@ __device__ __forceinline__ TaskBlock task_block(const int* map, int b) {
     return t;
 }
 
+// share [x, y) of worker w of `units` spread evenly over `workers`
+__device__ __forceinline__ int2 unit_share(int units, long long w, int workers) {
+    return make_int2((int)(w * units / workers), w < workers ? (int)((w + 1) * units / workers) : 0);
+}
+
 }  // namespace wema

@@ -653,12 +653,6 @@ __device__ __forceinline__ void guided_segment(const TransferParams& p, SweepRin
     }
 }
 
-// this warp's share of `units` spread evenly over `warps`
-__device__ __forceinline__ int2 unit_share(int units, int warps) {
-    const long long w = (long long)blockIdx.x * GS_WARPS + (threadIdx.x >> 5);
-    return make_int2((int)(w * units / warps), w < warps ? (int)((w + 1) * units / warps) : 0);
-}
-
 // ---- rows per segment, per device (the autotuner may change it): the default
 // splits the work evenly over the warps, any other height is fixed
 static std::atomic<int> g_seg_rows[64];
@@ -754,7 +748,7 @@ template <int MODE>
 __global__ void __launch_bounds__(GS_THREADS) k_guided_transfer(SpArgs args, int units, int warps) {
     __shared__ SweepRing rings[GS_WARPS];
     const int per = units_per_strip(args.p);
-    int2 u = unit_share(units, warps);
+    int2 u = unit_share(units, blockIdx.x * GS_WARPS + (threadIdx.x >> 5), warps);
     while (u.x < u.y) {
         const int strip = u.x / per, u0 = u.x - strip * per, n = min(u.y - u.x, per - u0);
         guided_segment<MODE>(args.p, rings[threadIdx.x >> 5], strip, u0, n);
@@ -772,7 +766,7 @@ template <int MODE>
 __global__ void __launch_bounds__(GS_THREADS, 6)
     k_guided_transfer_multi(const TransferParams* __restrict__ ps, const int* __restrict__ map, int warps) {
     __shared__ SweepRing rings[GS_WARPS];
-    int2 u = unit_share(map[1 + map[0]], warps);
+    int2 u = unit_share(map[1 + map[0]], blockIdx.x * GS_WARPS + (threadIdx.x >> 5), warps);
     while (u.x < u.y) {
         const TaskBlock t = task_block(map, u.x);       // x: unit in the strip, y: strip
         const TransferParams& p = ps[t.task];
