@@ -4,8 +4,8 @@
 // Each stream keeps its own state (a Session holding one buffer set: pyramid,
 // deltas, IIR state, threshold scratch and binade history) resident on the
 // device.  A tick takes one frame of each listed stream and issues, on one
-// CUDA stream, the same kernels as the per-stream path - forward DWT level 0
-// (luma and colour streams apart), levels 1..3, threshold monoids and walk,
+// CUDA stream, the same kernels as the per-stream path - forward DWT level 0,
+// levels 1..3, threshold monoids and walk,
 // the IIR filter (on a second CUDA stream, beside the threshold), inverse
 // levels 3..1, inverse level 0 and the luma transfer - but each launch covers
 // all streams: its grid is the concatenation of the streams' grids and a task
@@ -58,8 +58,8 @@ struct Launch {
     std::vector<int> gx, gy, nblk;
     unsigned total = 0;
     size_t params_off = 0, map_off = 0;   // device offsets in the tick's table
-    bool any16 = false;                   // some task has FP16 planes (planes_fp16)
-    int mode = -2;                        // guided transfer: the tasks' row form, -1 when they differ, -2 none
+    int kind = -2;                        // the tasks' common form (storage types; guided transfer: rows),
+                                          // -1 when they differ, -2 none
     void reset(size_t e) {
         elem = e;
         params.clear();
@@ -67,8 +67,7 @@ struct Launch {
         gy.clear();
         nblk.clear();
         total = 0;
-        any16 = false;
-        mode = -2;
+        kind = -2;
     }
     void add(const void* p, unsigned x, unsigned y, unsigned blocks) {
         if (blocks == 0) return;
@@ -79,10 +78,11 @@ struct Launch {
         total += blocks;
     }
     int n() const { return (int)gx.size(); }
+    void merge(int k) { kind = kind == -2 || kind == k ? k : -1; }
 };
 
 enum {
-    L_FWD0_LUMA, L_FWD0_COLOR, L_FWD1, L_FWD2, L_FWD3,
+    L_FWD0, L_FWD1, L_FWD2, L_FWD3,
     L_THR_PART, L_THR_PREFIX, L_THR_MON, L_THR_WALK, L_THR16,
     L_THR_MON0,                         // monoids of the level-0 sub-chunks, split off
     L_IIR_PRESEED, L_IIR,
@@ -476,9 +476,7 @@ public:
                 if (ids[q] == ids[k]) { set_error("stream %d listed twice in one tick", ids[k]); return false; }
         }
         for (auto& LG : L) {
-            LG[L_FWD0_LUMA].reset(sizeof(FwdLevelParams));
-            LG[L_FWD0_COLOR].reset(sizeof(FwdLevelParams));
-            for (int l = 1; l <= 3; l++) LG[L_FWD0_COLOR + l].reset(sizeof(FwdLevelParams));
+            for (int l = 0; l <= 3; l++) LG[L_FWD0 + l].reset(sizeof(FwdLevelParams));
             for (int k = L_THR_PART; k <= L_THR_MON0; k++) LG[k].reset(thr_args_bytes());
             LG[L_IIR_PRESEED].reset(iir_args_bytes());
             LG[L_IIR].reset(iir_args_bytes());
@@ -538,10 +536,10 @@ public:
                 p.prev_n = l > 0 ? g.n[l - 1] : 0;
                 if (S.frames_processed > 0) S.fill_temporal(p, l);   // the filter's step inside the transform
                 unsigned gx, gy;
-                Launch& lf = LK[l == 0 ? (nch == 3 ? L_FWD0_COLOR : L_FWD0_LUMA) : L_FWD0_COLOR + l];
-                const unsigned b = dwt_fwd_grid(p, l == 0 ? 1 : nch, gx, gy);
+                Launch& lf = LK[L_FWD0 + l];
+                const unsigned b = dwt_fwd_grid(p, nch, gx, gy);
                 lf.add(&p, gx, gy, b);
-                lf.any16 |= h;
+                lf.merge(dwt_fwd_kind(p));
             }
             // ---- threshold
             PyrView views[3];
@@ -602,9 +600,9 @@ public:
                 unsigned gx, gy;
                 if (l == 0 && nch == 3) iq.out_u8 = out[k];
                 Launch& li = LK[l == 0 ? (nch == 3 ? L_INV0_COLOR : L_INV0_LUMA) : L_INV1 - (l - 1)];
-                const unsigned b = dwt_inv_grid(iq, l == 0 && nch == 3 ? 1 : nch, l == 0 && nch == 3 ? kOutRgb : kOutPlanes, gx, gy);
+                const unsigned b = dwt_inv_grid(iq, l == 0 && nch == 3 ? 1 : nch, gx, gy);
                 li.add(&iq, gx, gy, b);
-                li.any16 |= iq.h16 != 0;
+                li.merge(iq.h16 != 0);
             }
             if (nch == 1) {
                 TransferParams tp{};
@@ -620,10 +618,7 @@ public:
                 const unsigned b = transfer_grid(tp, gx, gy);
                 Launch& lx = LK[tp.edge_aware ? L_XFER_GUIDED : L_XFER_GAUSS];
                 lx.add(&tp, gx, gy, b);
-                if (tp.edge_aware) {
-                    const int mode = transfer_rows_mode(tp);
-                    lx.mode = lx.mode == -2 || lx.mode == mode ? mode : -1;
-                }
+                if (tp.edge_aware) lx.merge(transfer_rows_mode(tp));
             }
         }
         // ---- the table image, its buffer, one H2D copy
@@ -671,12 +666,11 @@ public:
 
         // the stages of one group on one stream
         auto fwd0 = [&](int g, cudaStream_t st) {
-            return go(g, L_FWD0_LUMA, [&] { return launch_dwt_fwd_multi(kSrcRgbU8, 1, (const FwdLevelParams*)P(g, L_FWD0_LUMA), M(g, L_FWD0_LUMA), L[g][L_FWD0_LUMA].total, L[g][L_FWD0_LUMA].any16, st); }, "forward DWT") &&
-                   go(g, L_FWD0_COLOR, [&] { return launch_dwt_fwd_multi(kSrcRgbU8, 3, (const FwdLevelParams*)P(g, L_FWD0_COLOR), M(g, L_FWD0_COLOR), L[g][L_FWD0_COLOR].total, L[g][L_FWD0_COLOR].any16, st); }, "forward DWT");
+            return go(g, L_FWD0, [&] { return launch_dwt_fwd_multi(kSrcRgbU8, (const FwdLevelParams*)P(g, L_FWD0), M(g, L_FWD0), L[g][L_FWD0].total, L[g][L_FWD0].kind, st); }, "forward DWT");
         };
         auto fwdl = [&](int g, cudaStream_t st) {
             for (int k = L_FWD1; k <= L_FWD3; k++)
-                if (!go(g, k, [&] { return launch_dwt_fwd_multi(kSrcPlanes, 1, (const FwdLevelParams*)P(g, k), M(g, k), L[g][k].total, L[g][k].any16, st); }, "forward DWT"))
+                if (!go(g, k, [&] { return launch_dwt_fwd_multi(kSrcPlanes, (const FwdLevelParams*)P(g, k), M(g, k), L[g][k].total, L[g][k].kind, st); }, "forward DWT"))
                     return false;
             return true;
         };
@@ -702,16 +696,16 @@ public:
         };
         auto invl = [&](int g, cudaStream_t st) {
             for (int k = L_INV3; k <= L_INV1; k++)
-                if (!go(g, k, [&] { return launch_dwt_inv_multi(1, kOutPlanes, (const InvLevelParams*)P(g, k), M(g, k), L[g][k].total, L[g][k].any16, st); }, "inverse DWT"))
+                if (!go(g, k, [&] { return launch_dwt_inv_multi(1, kOutPlanes, (const InvLevelParams*)P(g, k), M(g, k), L[g][k].total, L[g][k].kind, st); }, "inverse DWT"))
                     return false;
             return true;
         };
         auto inv0 = [&](int g, cudaStream_t st) {
-            return go(g, L_INV0_LUMA, [&] { return launch_dwt_inv_multi(1, kOutPlanes, (const InvLevelParams*)P(g, L_INV0_LUMA), M(g, L_INV0_LUMA), L[g][L_INV0_LUMA].total, L[g][L_INV0_LUMA].any16, st); }, "inverse DWT") &&
-                   go(g, L_INV0_COLOR, [&] { return launch_dwt_inv_multi(3, kOutRgb, (const InvLevelParams*)P(g, L_INV0_COLOR), M(g, L_INV0_COLOR), L[g][L_INV0_COLOR].total, L[g][L_INV0_COLOR].any16, st); }, "inverse DWT");
+            return go(g, L_INV0_LUMA, [&] { return launch_dwt_inv_multi(1, kOutPlanes, (const InvLevelParams*)P(g, L_INV0_LUMA), M(g, L_INV0_LUMA), L[g][L_INV0_LUMA].total, L[g][L_INV0_LUMA].kind, st); }, "inverse DWT") &&
+                   go(g, L_INV0_COLOR, [&] { return launch_dwt_inv_multi(3, kOutRgb, (const InvLevelParams*)P(g, L_INV0_COLOR), M(g, L_INV0_COLOR), L[g][L_INV0_COLOR].total, L[g][L_INV0_COLOR].kind, st); }, "inverse DWT");
         };
         auto xfer = [&](int g, cudaStream_t st) {
-            return go(g, L_XFER_GUIDED, [&] { return launch_transfer_multi(1, (const TransferParams*)P(g, L_XFER_GUIDED), M(g, L_XFER_GUIDED), L[g][L_XFER_GUIDED].total, L[g][L_XFER_GUIDED].mode, st); }, "luma transfer") &&
+            return go(g, L_XFER_GUIDED, [&] { return launch_transfer_multi(1, (const TransferParams*)P(g, L_XFER_GUIDED), M(g, L_XFER_GUIDED), L[g][L_XFER_GUIDED].total, L[g][L_XFER_GUIDED].kind, st); }, "luma transfer") &&
                    go(g, L_XFER_GAUSS, [&] { return launch_transfer_multi(0, (const TransferParams*)P(g, L_XFER_GAUSS), M(g, L_XFER_GAUSS), L[g][L_XFER_GAUSS].total, 0, st); }, "luma transfer");
         };
         // a stage over every group in turn, between its timing marks
@@ -769,7 +763,7 @@ public:
                     sig.push_back(l.total);
                     sig.push_back((long long)l.params_off);
                     sig.push_back((long long)l.map_off);
-                    sig.push_back(l.any16 + 2 * l.mode);
+                    sig.push_back(l.kind);
                 }
             if (sig != t.sig) {
                 drop_graphs(t);

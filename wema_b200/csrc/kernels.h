@@ -32,6 +32,7 @@ struct FwdLevelParams {
     long long iir_off6;         // this level's first 6-slot index
     long long iir_simd_end;     // 6-slot indices from here take the scalar-tail form
     int iir_fp64;
+    int unit;                   // pairs of rows per unit of work (dwt_fwd_grid)
 };
 
 struct InvLevelParams {
@@ -48,18 +49,17 @@ struct InvLevelParams {
     float* out_f32;             // kOutRgb: float RGB output (optional)
     int h16;                    // coef and delta are FP16 planes (ll stays FP32)
     int out16;                  // out_planes are FP16 (the level-0 reconstruction of planes_fp16)
-    int unit;                   // planes out: pairs of rows per unit of work (filled in by the launch)
+    int unit;                   // pairs of rows per unit of work (dwt_inv_grid)
 };
 
 cudaError_t dwt_prepare_device();
-size_t dwt_smem_bytes(int channels);
 cudaError_t launch_dwt_fwd(int src_mode, int channels, const FwdLevelParams& p, cudaStream_t st);
 cudaError_t launch_dwt_inv(int channels, int out_mode, const InvLevelParams& p, cudaStream_t st);
-// tuning variant (0..8) of the batched luma DWT kernels on a device:
-// CTAs per SM {1: the compiler's choice, 3, 4}[v / 3] x lines per warp {2, 4, 8}[v % 3]
+// tuning variant (0..8) of the DWT sweeps on a device: at most {3, 4, 5}[v / 3]
+// CTAs per SM, units of {1, 2, 4}[v % 3] pairs of rows
 int dwt_variant(int dev, int inverse);
 bool dwt_set_variant(int dev, int inverse, int v);
-void dwt_variant_shape(int v, int* minb, int* lpw);
+void dwt_variant_shape(int v, int* res, int* unit);
 // times every variant of the forward and inverse level-0 luma kernels, keeps the fastest
 cudaError_t dwt_autotune(int dev, float fwd_ms[9], float inv_ms[9], int* fwd_best, int* inv_best);
 
@@ -158,14 +158,14 @@ cudaError_t launch_window(const WindowParams& wp, int channels, cudaStream_t st)
 // ---- batched launches: one launch of a kernel over many streams --------------
 // Every launch takes a device array of per-task parameters and a task map
 // (multi.cuh); `blocks` is the sum of the tasks' grids.
-unsigned dwt_fwd_grid(const FwdLevelParams& p, int channels_z, unsigned& gx, unsigned& gy);
-unsigned dwt_inv_grid(InvLevelParams& p, int channels_z, int out_mode, unsigned& gx, unsigned& gy);
-// any16: some task has FP16 planes (planes_fp16); false selects the kernel
-// compiled for FP32 planes only
-cudaError_t launch_dwt_fwd_multi(int mode, int channels, const FwdLevelParams* d_params,
-                                 const int* d_map, unsigned blocks, bool any16, cudaStream_t st);
+unsigned dwt_fwd_grid(FwdLevelParams& p, int channels_z, unsigned& gx, unsigned& gy);
+unsigned dwt_inv_grid(InvLevelParams& p, int channels_z, unsigned& gx, unsigned& gy);
+// kind: the tasks' common dwt_fwd_kind (inverse: h16), or -1 when they differ
+int dwt_fwd_kind(const FwdLevelParams& p);
+cudaError_t launch_dwt_fwd_multi(int mode, const FwdLevelParams* d_params, const int* d_map, unsigned blocks, int kind,
+                                 cudaStream_t st);
 cudaError_t launch_dwt_inv_multi(int channels, int out_mode, const InvLevelParams* d_params,
-                                 const int* d_map, unsigned blocks, bool any16, cudaStream_t st);
+                                 const int* d_map, unsigned blocks, int kind, cudaStream_t st);
 size_t thr_args_bytes();
 // grids[stage] = {x, y} for stage 0 partials, 1 prefix, 2 monoids, 3 walk
 cudaError_t thr_args_fill(void* dst, const PyrView* views, int nch, const ThrScratch* scratch,

@@ -745,7 +745,7 @@ WEMA_API int wema_cuda_autotune(int device, char* report, size_t cap) {
                          ms[0], ms[1], ms[2], chosen, gms[0], gms[1], gms[2], grows);
         for (int inv = 0; inv < 2 && n > 0 && (size_t)n < cap; inv++) {
             const float* t = inv ? ims : fms;
-            n += snprintf(report + n, cap - n, "; %s DWT level 0 (CTAs/SM x lines/warp):",
+            n += snprintf(report + n, cap - n, "; %s DWT level 0 (CTAs/SM x pairs of rows):",
                           inv ? "inverse" : "forward");
             for (int v = 0; v < 9 && n > 0 && (size_t)n < cap; v++) {
                 int mb, lp;

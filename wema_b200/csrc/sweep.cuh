@@ -56,13 +56,9 @@ __device__ __forceinline__ int mirror(int i, int n) {
     return i < n ? i : p - i;
 }
 
-// Asynchronous copies of a lane's own elements into its own slots of shared
-// memory: only the copying thread reads them, after its own wait, so a ring of
-// them needs no barrier.
-template <int BYTES>
-__device__ __forceinline__ void cp_async(void* dst, const void* src) {
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
