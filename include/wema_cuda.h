@@ -307,11 +307,11 @@ int wema_cuda_server_stats(wema_cuda_server *srv, int reset, wema_cuda_serve_sta
  *     warps (the setting 64, the default) and at 128 and 256 output rows per
  *     segment (a 3840x8640 trial frame) and keeps the fastest;
  *   - the batched luma DWT level-0 kernels, forward and inverse, in nine
- *     variants each: CTAs per SM asked of the register allocator {1 (the
- *     compiler's choice), 3, 4} x lines lifted per warp at a time {2, 4, 8}
- *     (variant = 3 * index + index; a 3840x4320 trial frame, the forward
- *     with the temporal filter's step inside as steady batched ticks run it)
- *     and keeps the fastest of each (4x4 for both until then);
+ *     variants each: at most {3, 4, 5} CTAs per SM (fewer where fewer fit) x
+ *     units of {1, 2, 4} pairs of rows (variant = 3 * index + index; a
+ *     3840x4320 trial frame, the forward with the temporal filter's step
+ *     inside as steady batched ticks run it) and keeps the fastest of each
+ *     (5 x 2 for both until then);
  * allocating ~950 MB for the trials (one at a time) and freeing it.  Every
  * later launch on the device uses the choices.  Returns the positions per
  * thread (or -1) and writes the timings to `report` (may be NULL; 1 KiB is

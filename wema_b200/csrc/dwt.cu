@@ -14,9 +14,13 @@
 // separate multiplies (dwt.c:45-170 as GCC -Ofast evaluates it), so
 // coefficients are bit-exact.
 //
-// What bounds them: HBM at the large levels (level 0 of the 48-stream tick:
-// forward see k_dwt_fwd, inverse see k_dwt_inv), the chain of steps of a short
-// segment at the small ones.
+// What bounds them: HBM and issue slots at the large levels, the chain of steps of
+// a short segment at the small ones.  Measured against kernels that staged
+// 64x64 regions in shared memory and wrote 54x54 of them (1.4 times the area,
+// 80 instructions per pixel of the inverse against 32 here):
+//   3840x4320, level 0   forward 55 -> 37 us (bytes in, planes out), with the
+//                        filter's step 140 -> 118; inverse 55 -> 41
+//   the 48-stream tick   inverse level 0 279 -> 173 us, levels 3..1 116 -> 81
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
@@ -182,6 +186,11 @@ __device__ __forceinline__ void st_pair(float* p, int i, const float (&v)[SQ], b
     }
 }
 
+// an element that the same launch may have written (the levels of k_dwt_fwd_tail)
+__device__ __forceinline__ float pl_ldcg(const float* p, int i, bool h) {
+    return h ? __half2float(__ldcg(reinterpret_cast<const __half*>(p) + i)) : __ldcg(p + i);
+}
+
 // Write-out of a lane's SQ positions of row y of one channel: LL, the bands LH,
 // HH, HL (v[0..2]), and the temporal filter's step on them (cascade.cuh): the
 // filter reads the coefficient as stored (FP16-rounded in the planes_fp16
@@ -305,9 +314,9 @@ __device__ __forceinline__ void fwd_sweep(const FwdSweep<MODE, H16, F64>& p, Row
                 const bool hx = !EDGE || 2 * (g + k) + 1 < p.iw;
                 const int at = y * p.sw + g + k;
                 if (k && !second) break;
-                if (!hy) v[0][k] = pv ? pl_ld(pv, at, H16) : 0.0f;
-                if (!(hx && hy)) v[1][k] = pv ? pl_ld(pv, pn + at, H16) : 0.0f;
-                if (!hx) v[2][k] = pv ? pl_ld(pv, 2 * pn + at, H16) : 0.0f;
+                if (!hy) v[0][k] = pv ? pl_ldcg(pv, at, H16) : 0.0f;
+                if (!(hx && hy)) v[1][k] = pv ? pl_ldcg(pv, pn + at, H16) : 0.0f;
+                if (!hx) v[2][k] = pv ? pl_ldcg(pv, 2 * pn + at, H16) : 0.0f;
             }
         }
         const bool tail = p.g.iir_off6 + 2 * p.n + (long long)y * p.sw + s.p0 + s.hi > p.g.iir_simd_end;
@@ -371,26 +380,33 @@ struct InvSweep {
 // SQ neighbouring elements of a plane as they were loaded: FP16 ones packed in
 // w[0] (a vector load) or one by one, widened when they are used, a pair of rows
 // later
-template <bool H16>
+// FRESH: the same launch may have written them (the levels of k_dwt_inv_tail):
+// not through the read-only path
+template <bool H16, bool FRESH = false>
 struct Elems {
     float w[SQ];
+    template <class T>
+    static __device__ __forceinline__ T ld(const T* p) {
+        if constexpr (FRESH) return __ldcg(p);
+        else return __ldg(p);
+    }
     __device__ __forceinline__ void load(const float* p, int i, bool vec, int n) {
         if (H16) {
             const __half* q = reinterpret_cast<const __half*>(p) + i;
             if (vec) {
-                w[0] = __ldg(reinterpret_cast<const float*>(q));
+                w[0] = ld(reinterpret_cast<const float*>(q));
             } else {
 #pragma unroll
                 for (int k = 0; k < SQ; k++)
-                    if (k < n) w[k] = __uint_as_float(__ldg(reinterpret_cast<const unsigned short*>(q + k)));
+                    if (k < n) w[k] = __uint_as_float(ld(reinterpret_cast<const unsigned short*>(q + k)));
             }
         } else if (vec) {
-            const float2 a = __ldg(reinterpret_cast<const float2*>(p + i));
+            const float2 a = ld(reinterpret_cast<const float2*>(p + i));
             w[0] = a.x; w[1] = a.y;
         } else {
 #pragma unroll
             for (int k = 0; k < SQ; k++)
-                if (k < n) w[k] = __ldg(p + i + k);
+                if (k < n) w[k] = ld(p + i + k);
         }
     }
     __device__ __forceinline__ void get(bool vec, float (&v)[SQ]) const {
@@ -407,9 +423,9 @@ struct Elems {
 
 // The loads of one pair of rows: LL and the three bands (LH, HH, HL) with their
 // deltas, per channel.
-template <int C, bool H16>
+template <int C, bool H16, bool FRESH>
 struct InvRows {
-    Elems<false> ll[C];
+    Elems<false, FRESH> ll[C];
     Elems<H16> x[C][3], d[C][3];
 
     // row pair j; g: the lane's first pair
@@ -451,7 +467,7 @@ __device__ __forceinline__ void put_samples(float* out, int at, int left, bool v
     }
 }
 
-template <int C, int OUT, bool H16, bool EDGE>
+template <int C, int OUT, bool H16, bool EDGE, bool FRESH = false>
 __device__ __forceinline__ void inv_sweep(const InvSweep<C, H16>& p, const Strip<SQ>& s, int ya, int yb) {
     const int lane = threadIdx.x & 31;
     const int g = s.p0 + SQ * lane;
@@ -466,7 +482,7 @@ __device__ __forceinline__ void inv_sweep(const InvSweep<C, H16>& p, const Strip
             L[c].o0[k] = L[c].e1[k] = L[c].o1[k] = L[c].e2[k] = 0.0f;
             H[c].o0[k] = H[c].e1[k] = H[c].o1[k] = H[c].e2[k] = 0.0f;
         }
-    InvRows<C, H16> r;
+    InvRows<C, H16, FRESH> r;
     const int j1 = yb + 2;
     r.issue(p, ya - 2, g);
 #pragma unroll 1
@@ -599,6 +615,58 @@ __global__ void __launch_bounds__(SW_THREADS, inv_res(C)) k_dwt_inv(const __grid
     each_segment(units, (g.sh + g.unit - 1) / g.unit, groups_of(g.sw), [&](int row, int group, int z, int n) {
         inv_segment<C, OUT, H16>(InvSweep<C, H16>(g, z), group, row, n);
     });
+}
+
+// The coarser levels of a small frame in one launch: a cluster per channel takes
+// them in turn, with a cluster barrier between two levels.  Warps of a sweep do not
+// meet, so each takes an even share of a level's rows of strips.
+// What bounds it: the chain of a warp's steps (rows + 4 of them at each level); a
+// level of few rows launched apart costs more than that in the host's launch
+// (about 2.5 us) and the wait for the kernel before.  12 warps: the rings' 38 KB.
+constexpr int TAIL_CTAS = 8, TAIL_WARPS = 12;
+template <class P>
+struct LevelTail {
+    P lv[3];                             // in the order they run
+    int count;
+};
+// f(strip, first pair of rows, end) for each of this warp's shares
+template <class F>
+__device__ __forceinline__ void tail_shares(int sw, int sh, F f) {
+    const int strips = (sw + SW_LANES * SQ - 1) / (SW_LANES * SQ);
+    int2 u = unit_share(strips * sh, blockIdx.x * TAIL_WARPS + (threadIdx.x >> 5), TAIL_CTAS * TAIL_WARPS);
+    while (u.x < u.y) {
+        const int s = u.x / sh, y = u.x % sh, n = min(u.y - u.x, sh - y);
+        f(Strip<SQ>(s, sw), y, y + n);
+        u.x += n;
+    }
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+template <bool H16>
+__global__ void __cluster_dims__(TAIL_CTAS, 1, 1) __launch_bounds__(32 * TAIL_WARPS)
+    k_dwt_fwd_tail(const __grid_constant__ LevelTail<FwdLevelParams> t) {
+    __shared__ RowRing<kSrcPlanes> rows[TAIL_WARPS];
+#pragma unroll 1
+    for (int l = 0; l < t.count; l++) {
+        if (l) cluster_barrier();
+        const FwdSweep<kSrcPlanes, H16, false> p(t.lv[l], blockIdx.y);
+        tail_shares(p.sw, p.sh, [&](const Strip<SQ>& s, int ya, int yb) {
+            fwd_sweep<kSrcPlanes, H16, false, true>(p, rows[threadIdx.x >> 5], nullptr, s, ya, yb);
+        });
+    }
+}
+template <bool H16>
+__global__ void __cluster_dims__(TAIL_CTAS, 1, 1) __launch_bounds__(32 * TAIL_WARPS)
+    k_dwt_inv_tail(const __grid_constant__ LevelTail<InvLevelParams> t) {
+#pragma unroll 1
+    for (int l = 0; l < t.count; l++) {
+        if (l) cluster_barrier();
+        const InvSweep<1, H16> p(t.lv[l], blockIdx.y);
+        tail_shares(p.sw, p.sh, [&](const Strip<SQ>& s, int ya, int yb) {
+            inv_sweep<1, kOutPlanes, H16, true, true>(p, s, ya, yb);
+        });
+    }
 }
 // batched (task = stream; params in device memory, one entry per task): the map
 // counts units
@@ -787,6 +855,49 @@ cudaError_t launch_dwt_inv(int channels, int out_mode, const InvLevelParams& p0,
     else if (out_mode == kOutRgb && channels == 3) go_inv<3, kOutRgb>(p, units, st);
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
+}
+
+// Whether levels from one of sw x sh positions on run in a cluster: at most 6 rows
+// of a strip per warp.  A stream's frame, levels apart -> in a cluster: 320x240
+// (1.2 rows) 49 -> 43 us, colour 42 -> 36; 853x479 (5.0) 64 -> 59, colour
+// 65 -> 56; 1023x577 (7.6) 63 -> 65, colour 66 -> 72; 1920x1080 (22.5) 82 -> 98:
+// from about 7 rows on the whole GPU is faster than a cluster's 8 SMs.
+constexpr int TAIL_ROWS = 6;
+static bool tail_fits(int sw, int sh, int n) {
+    const long long rows = (long long)((sw + SW_LANES * SQ - 1) / (SW_LANES * SQ)) * sh;
+    return n >= 2 && n <= 3 && rows <= TAIL_ROWS * TAIL_CTAS * TAIL_WARPS;
+}
+cudaError_t launch_dwt_fwd_levels(int channels, const FwdLevelParams* p, int n, cudaStream_t st, int* launches) {
+    if (n > 0 && tail_fits(p[0].sw, p[0].sh, n)) {
+        LevelTail<FwdLevelParams> t{};
+        for (int l = 0; l < n; l++) t.lv[l] = p[l];
+        t.count = n;
+        const dim3 grid(TAIL_CTAS, (unsigned)channels);
+        if (p[0].h16) k_dwt_fwd_tail<true><<<grid, 32 * TAIL_WARPS, 0, st>>>(t);
+        else k_dwt_fwd_tail<false><<<grid, 32 * TAIL_WARPS, 0, st>>>(t);
+        *launches = 1;
+        return cudaGetLastError();
+    }
+    *launches = n;
+    cudaError_t e = cudaSuccess;
+    for (int l = 0; l < n && e == cudaSuccess; l++) e = launch_dwt_fwd(kSrcPlanes, channels, p[l], st);
+    return e;
+}
+cudaError_t launch_dwt_inv_levels(int channels, const InvLevelParams* p, int n, cudaStream_t st, int* launches) {
+    if (n > 0 && tail_fits(p[n - 1].sw, p[n - 1].sh, n)) {
+        LevelTail<InvLevelParams> t{};
+        for (int l = 0; l < n; l++) t.lv[l] = p[l];
+        t.count = n;
+        const dim3 grid(TAIL_CTAS, (unsigned)channels);
+        if (p[0].h16) k_dwt_inv_tail<true><<<grid, 32 * TAIL_WARPS, 0, st>>>(t);
+        else k_dwt_inv_tail<false><<<grid, 32 * TAIL_WARPS, 0, st>>>(t);
+        *launches = 1;
+        return cudaGetLastError();
+    }
+    *launches = n;
+    cudaError_t e = cudaSuccess;
+    for (int l = 0; l < n && e == cudaSuccess; l++) e = launch_dwt_inv(channels, kOutPlanes, p[l], st);
+    return e;
 }
 
 }  // namespace wema

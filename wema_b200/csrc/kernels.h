@@ -55,6 +55,10 @@ struct InvLevelParams {
 cudaError_t dwt_prepare_device();
 cudaError_t launch_dwt_fwd(int src_mode, int channels, const FwdLevelParams& p, cudaStream_t st);
 cudaError_t launch_dwt_inv(int channels, int out_mode, const InvLevelParams& p, cudaStream_t st);
+// n consecutive levels after the first (forward: finest first, inverse: coarsest
+// first), planes in and out; *launches: how many it took
+cudaError_t launch_dwt_fwd_levels(int channels, const FwdLevelParams* p, int n, cudaStream_t st, int* launches);
+cudaError_t launch_dwt_inv_levels(int channels, const InvLevelParams* p, int n, cudaStream_t st, int* launches);
 // tuning variant (0..8) of the DWT sweeps on a device: at most {3, 4, 5}[v / 3]
 // CTAs per SM, units of {1, 2, 4}[v % 3] pairs of rows
 int dwt_variant(int dev, int inverse);

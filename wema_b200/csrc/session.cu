@@ -330,8 +330,10 @@ bool Session::run(const uint8_t* in_u8, const float* in_f32, uint8_t* out_u8, fl
 
     // ---- forward DWT
     mark(2 * ST_FWD0, s_fwd);
+    FwdLevelParams fp[WEMA_MAX_LEV]{};
+    int used = 0;
     for (int l = 0; l < L; l++) {
-        FwdLevelParams p{};
+        FwdLevelParams& p = fp[l];
         p.iw = g.in_w[l];
         p.ih = g.in_h[l];
         p.sw = g.sw[l];
@@ -356,13 +358,15 @@ bool Session::run(const uint8_t* in_u8, const float* in_f32, uint8_t* out_u8, fl
         }
         p.prev_n = l > 0 ? g.n[l - 1] : 0;
         p.h16 = h;
-        if (!cuda_ok(launch_dwt_fwd(mode, nch, p, s_fwd), "forward DWT")) return false;
-        launches++;
         if (l == 0) {
+            if (!cuda_ok(launch_dwt_fwd(mode, nch, p, s_fwd), "forward DWT")) return false;
+            launches++;
             mark(2 * ST_FWD0 + 1, s_fwd);
             mark(2 * ST_FWD, s_fwd);
         }
     }
+    if (!cuda_ok(launch_dwt_fwd_levels(nch, fp + 1, L - 1, s_fwd, &used), "forward DWT")) return false;
+    launches += used;
     mark(2 * ST_FWD + 1, s_fwd);
     if (!cuda_ok(cudaEventRecord(q.ev_fwd, s_fwd), "event record")) return false;
 
@@ -462,8 +466,9 @@ bool Session::run(const uint8_t* in_u8, const float* in_f32, uint8_t* out_u8, fl
         launches++;
     } else {
         mark(2 * ST_INV, s_inv);
+        InvLevelParams lv[WEMA_MAX_LEV]{};   // coarsest first
         for (int l = L - 1; l >= 0; l--) {
-            InvLevelParams iq{};
+            InvLevelParams& iq = lv[L - 1 - l];
             iq.ow = g.in_w[l];
             iq.oh = g.in_h[l];
             iq.sw = g.sw[l];
@@ -481,6 +486,8 @@ bool Session::run(const uint8_t* in_u8, const float* in_f32, uint8_t* out_u8, fl
                 iq.out_planes[c] = (l > 0 || nch == 1 || inspect) ? q.rec[c][l] : nullptr;
             }
             if (l == 0) {
+                if (!cuda_ok(launch_dwt_inv_levels(nch, lv, L - 1, s_inv, &used), "inverse DWT")) return false;
+                launches += used;
                 mark(2 * ST_INV + 1, s_inv);
                 mark(2 * ST_INV0, s_inv);
             }
@@ -490,8 +497,10 @@ bool Session::run(const uint8_t* in_u8, const float* in_f32, uint8_t* out_u8, fl
                 iq.out_u8 = out_u8;
                 iq.out_f32 = out_f32;
             }
-            if (!cuda_ok(launch_dwt_inv(nch, mode, iq, s_inv), "inverse DWT")) return false;
-            launches++;
+            if (l == 0) {
+                if (!cuda_ok(launch_dwt_inv(nch, mode, iq, s_inv), "inverse DWT")) return false;
+                launches++;
+            }
         }
         mark(2 * ST_INV0 + 1, s_inv);
         mark(2 * ST_XFER, s_inv);

@@ -8,7 +8,7 @@
 // the lifting keeps its last value, so a pair of rows that enters moves every
 // step on by one and a finished pair of rows, two behind, comes out.
 // There is no staging, no block barrier and no shared memory but the forward's
-// write-out buffer.
+// rings of incoming rows and state, which are a warp's own.
 //
 // Every output depends on samples within 4 of it.  Strips overlap by one
 // lane on either side (30 lanes write; the garbage that lane 0 and lane 31 take
