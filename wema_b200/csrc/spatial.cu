@@ -550,10 +550,13 @@ __device__ __forceinline__ void guided_sweep(const TransferParams& pg, SweepRing
                 const float inv = __fmul_rn(icx[j], icy);
                 const float mI = __fmul_rn(sI[j], inv), mP = __fmul_rn(sP[j], inv);
                 const float cII = __fmul_rn(sII[j], inv), cIP = __fmul_rn(sIP[j], inv);
-                // the denominator is >= eps + E[I^2] - E[I]^2 > 0; a within 2 ulp.
-                // Outside the image inv and so every mean is 0: a = b = 0
-                a[j] = div_normal(__fmaf_rn(-mI, mP, cIP), __fmaf_rn(-mI, mI, __fadd_rn(cII, kEps)));
-                b[j] = __fmaf_rn(-a[j], mI, mP);
+                // the denominator is >= eps + E[I^2] - E[I]^2 > 0; a within 2 ulp
+                const float av = div_normal(__fmaf_rn(-mI, mP, cIP), __fmaf_rn(-mI, mI, __fadd_rn(cII, kEps)));
+                // outside the image 0 by selection: a sum that overflowed would make
+                // its product with inv = 0 a NaN, which the windows inside would take in
+                const bool inside = inv != 0.f;
+                a[j] = inside ? av : 0.f;
+                b[j] = inside ? __fmaf_rn(-av, mI, mP) : 0.f;
             }
         }
         // second round: horizontal sums of a, b into the ring; vertical sums over rows c1-8..c1
