@@ -138,13 +138,6 @@ __device__ __forceinline__ void hwin(const float v[4], float o[4]) {
     }
 }
 
-// a / b for a normal b > 0: the fast division's product with the reciprocal
-// without its rescaling of denormal or huge b
-__device__ __forceinline__ float div_normal(float a, float b) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
-    return __fmul_rn(a, r);
-}
 __device__ __forceinline__ float max_nan(float a, float b) {   // NaN if either is
     float r;
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
@@ -551,7 +544,7 @@ __device__ __forceinline__ void guided_sweep(const TransferParams& pg, SweepRing
                 const float mI = __fmul_rn(sI[j], inv), mP = __fmul_rn(sP[j], inv);
                 const float cII = __fmul_rn(sII[j], inv), cIP = __fmul_rn(sIP[j], inv);
                 // the denominator is >= eps + E[I^2] - E[I]^2 > 0; a within 2 ulp
-                const float av = div_normal(__fmaf_rn(-mI, mP, cIP), __fmaf_rn(-mI, mI, __fadd_rn(cII, kEps)));
+                const float av = __fdividef(__fmaf_rn(-mI, mP, cIP), __fmaf_rn(-mI, mI, __fadd_rn(cII, kEps)));
                 // outside the image 0 by selection: a sum that overflowed would make
                 // its product with inv = 0 a NaN, which the windows inside would take in
                 const bool inside = inv != 0.f;
