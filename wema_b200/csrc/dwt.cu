@@ -29,6 +29,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "multi.cuh"
+#include "row_copy.h"
 #include "sweep.cuh"
 
 namespace wema {
@@ -36,6 +37,21 @@ namespace wema {
 constexpr int SQ = 2;                    // pairs of columns per lane
 
 // ----------------------------------------------------------------- forward
+// A warp's inputs of FWD_RING consecutive pairs of rows in shared memory, copied
+// in asynchronously FWD_RING - 1 ahead in whole 16-byte pieces: the strip's part
+// of the two rows, and the temporal filter's state of the row of positions that
+// the step finishes.
+constexpr int FWD_RING = 3;
+template <int MODE>
+struct RowRing {
+    static constexpr int PX = MODE == kSrcRgbU8 ? 3 : MODE == kSrcRgbF32 ? 12 : 4;   // bytes per sample
+    static constexpr int PIECES = 64 * SQ * PX / 16 + 1;                             // one more: any alignment
+    uint4 v[FWD_RING][2][PIECES];
+};
+struct StateRing {
+    float4 v[FWD_RING][3][32 * SQ];
+};
+
 // What a sweep of channel z of a level uses of its parameters; what it rarely
 // uses stays in g.  F64: the biquad state and its update in FP64.  (A colour
 // frame's three channels are swept apart, each converting the pixels to its
@@ -45,6 +61,7 @@ template <int MODE, bool H16, bool F64>
 struct FwdSweep {
     const FwdLevelParams& g;
     int z, iw, ih, sw, sh, n, unit, vec_end;
+    int inner;                           // rows whose copies may be whole pieces (row_copy.h)
     const void* src;                     // RGB24, float RGB, or the channel's plane
     float *coef, *ll, *dl;
     void* st;
@@ -56,6 +73,7 @@ struct FwdSweep {
     }
     __device__ __forceinline__ FwdSweep(const FwdLevelParams& g_, int z_)
         : g(g_), z(z_), iw(g.iw), ih(g.ih), sw(g.sw), sh(g.sh), n((int)g.n), unit(g.unit), vec_end((int)g.vec_end) {
+        inner = inner_rows(ih, RowRing<MODE>::PX * iw);
         coef = pick(g.coef);
         ll = pick(g.ll_out);
         dl = pick(g.iir_delta);
@@ -71,36 +89,34 @@ struct FwdSweep {
     }
 };
 
-// A warp's inputs of FWD_RING consecutive pairs of rows in shared memory, copied
-// in asynchronously FWD_RING - 1 ahead in whole 16-byte pieces: the strip's part
-// of the two rows, and the temporal filter's state of the row of positions that
-// the step finishes.
-constexpr int FWD_RING = 3;
-template <int MODE>
-struct RowRing {
-    static constexpr int PX = MODE == kSrcRgbU8 ? 3 : MODE == kSrcRgbF32 ? 12 : 4;   // bytes per sample
-    static constexpr int PIECES = 64 * SQ * PX / 16 + 1;                             // one more: any alignment
-    uint4 v[FWD_RING][2][PIECES];
-};
-struct StateRing {
-    float4 v[FWD_RING][3][32 * SQ];
-};
 // the address of the strip's first sample of image row `row`
 template <int MODE, class S>
 __device__ __forceinline__ const uint8_t* row_start(const S& p, int row, int p0) {
     return static_cast<const uint8_t*>(p.src) + (long long)RowRing<MODE>::PX * (row * p.iw + 2 * p0);
 }
-// the strip's part of row h of pair j (a 16-byte piece that holds a byte of the
-// frame is mapped memory, even where it reaches past the frame's ends)
+// a row's part in 4-byte words, where 16-byte pieces may reach past the frame; out
+// of line, as only the frame's first and last rows come here
+__device__ __noinline__ void row_words(uint8_t* d, const uint8_t* q, int bytes) {
+    const int off = (int)(reinterpret_cast<uintptr_t>(q) & 15), at = off & ~3;
+    const int words = (off - at + bytes + 3) >> 2;
+    for (int k = threadIdx.x & 31; k < words; k += 32) cp_async4(d + at + 4 * k, q - off + at + 4 * k);
+}
+// the strip's part of the two rows of pair j (a plane lies in the library's own
+// memory, on either side of it too)
 template <int MODE, class S>
 __device__ __forceinline__ void row_issue(const S& p, RowRing<MODE>& ring, int slot, int j, int p0) {
     const int bytes = RowRing<MODE>::PX * min(64 * SQ, p.iw - 2 * p0);
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        const uint8_t* q = row_start<MODE>(p, mirror(2 * j + h, p.ih), p0);
-        const int off = (int)(reinterpret_cast<uintptr_t>(q) & 15);
-        const int pieces = (off + bytes + 15) >> 4;
-        for (int k = threadIdx.x & 31; k < pieces; k += 32) cp_async16(&ring.v[slot][h][k], q - off + 16 * k);
+        const int row = mirror(2 * j + h, p.ih);
+        const uint8_t* q = row_start<MODE>(p, row, p0);
+        if (MODE == kSrcPlanes || row_inner(row, p.inner)) {   // (uniform)
+            const int off = (int)(reinterpret_cast<uintptr_t>(q) & 15);
+            const int pieces = (off + bytes + 15) >> 4;
+            for (int k = threadIdx.x & 31; k < pieces; k += 32) cp_async16(&ring.v[slot][h][k], q - off + 16 * k);
+        } else {
+            row_words(reinterpret_cast<uint8_t*>(ring.v[slot][h]), q, bytes);
+        }
     }
 }
 // the samples of row h of the pair
