@@ -58,7 +58,7 @@ struct Launch {
     std::vector<int> gx, gy, nblk;
     unsigned total = 0;
     size_t params_off = 0, map_off = 0;   // device offsets in the tick's table
-    int kind = -2;                        // the tasks' common form (storage types; guided transfer: rows),
+    int kind = -2;                        // the tasks' common form (transforms: kDwt..., guided transfer: rows),
                                           // -1 when they differ, -2 none
     void reset(size_t e) {
         elem = e;
@@ -82,7 +82,8 @@ struct Launch {
 };
 
 enum {
-    L_FWD0, L_FWD1, L_FWD2, L_FWD3,
+    L_FWD0, L_FWD0_COLOR,               // (colour apart by tiles only)
+    L_FWD1, L_FWD2, L_FWD3,
     L_THR_PART, L_THR_PREFIX, L_THR_MON, L_THR_WALK, L_THR16,
     L_THR_MON0,                         // monoids of the level-0 sub-chunks, split off
     L_IIR_PRESEED, L_IIR,
@@ -476,7 +477,7 @@ public:
                 if (ids[q] == ids[k]) { set_error("stream %d listed twice in one tick", ids[k]); return false; }
         }
         for (auto& LG : L) {
-            for (int l = 0; l <= 3; l++) LG[L_FWD0 + l].reset(sizeof(FwdLevelParams));
+            for (int k = L_FWD0; k <= L_FWD3; k++) LG[k].reset(sizeof(FwdLevelParams));
             for (int k = L_THR_PART; k <= L_THR_MON0; k++) LG[k].reset(thr_args_bytes());
             LG[L_IIR_PRESEED].reset(iir_args_bytes());
             LG[L_IIR].reset(iir_args_bytes());
@@ -508,9 +509,30 @@ public:
             }
         }
 
+        // The transforms' form, per group: sweeps where the streams agree in storage
+        // type and hold no FP64 state, else tiles.  A kernel of sweeps for every type
+        // spills, and the FP64 state's loads need more warps than sweeps have: eight
+        // 1280x720 streams per tick, sweeps -> tiles: state_fp64 391 -> 357 us, a mix
+        // of the variants 422 -> 358, in colour 837 -> 620.
+        int fform[MAXG], iform[MAXG];
+        for (int g = 0; g < G; g++) {
+            bool some16 = false, all16 = true, wide = false;
+            for (int k = 0; k < n; k++) {
+                if (grp[k] != g) continue;
+                const Session& S = *streams[ids[k]];
+                some16 |= S.cfg.planes_fp16 != 0;
+                all16 &= S.cfg.planes_fp16 != 0;
+                wide |= S.frames_processed > 0 && S.cfg.iir_state_fp64;
+            }
+            const int tiles = some16 ? kDwtTiles16 : kDwtTiles, sweep = some16 ? kDwtSweep16 : kDwtSweep;
+            fform[g] = wide || some16 != all16 ? tiles : sweep;
+            iform[g] = some16 != all16 ? tiles : sweep;
+        }
+
         for (const int k : order) {
             Session& S = *streams[ids[k]];
             Launch* const LK = L[grp[k]];
+            const int ff = fform[grp[k]], fi = iform[grp[k]];
             const Geom& g = S.g;
             const int LV = g.levels, nch = S.nch;
             Slot& q = S.slot[0];
@@ -536,10 +558,11 @@ public:
                 p.prev_n = l > 0 ? g.n[l - 1] : 0;
                 if (S.frames_processed > 0) S.fill_temporal(p, l);   // the filter's step inside the transform
                 unsigned gx, gy;
-                Launch& lf = LK[L_FWD0 + l];
-                const unsigned b = dwt_fwd_grid(p, nch, gx, gy);
+                const bool apart = l == 0 && ff >= kDwtTiles;
+                Launch& lf = LK[l > 0 ? L_FWD1 + (l - 1) : apart && nch == 3 ? L_FWD0_COLOR : L_FWD0];
+                const unsigned b = dwt_fwd_grid(p, apart ? 1 : nch, ff, gx, gy);
                 lf.add(&p, gx, gy, b);
-                lf.merge(dwt_fwd_kind(p));
+                lf.merge(ff);
             }
             // ---- threshold
             PyrView views[3];
@@ -600,9 +623,9 @@ public:
                 unsigned gx, gy;
                 if (l == 0 && nch == 3) iq.out_u8 = out[k];
                 Launch& li = LK[l == 0 ? (nch == 3 ? L_INV0_COLOR : L_INV0_LUMA) : L_INV1 - (l - 1)];
-                const unsigned b = dwt_inv_grid(iq, l == 0 && nch == 3 ? 1 : nch, gx, gy);
+                const unsigned b = dwt_inv_grid(iq, l == 0 && nch == 3 ? 1 : nch, fi, gx, gy);
                 li.add(&iq, gx, gy, b);
-                li.merge(iq.h16 != 0);
+                li.merge(fi);
             }
             if (nch == 1) {
                 TransferParams tp{};
@@ -666,11 +689,12 @@ public:
 
         // the stages of one group on one stream
         auto fwd0 = [&](int g, cudaStream_t st) {
-            return go(g, L_FWD0, [&] { return launch_dwt_fwd_multi(kSrcRgbU8, (const FwdLevelParams*)P(g, L_FWD0), M(g, L_FWD0), L[g][L_FWD0].total, L[g][L_FWD0].kind, st); }, "forward DWT");
+            return go(g, L_FWD0, [&] { return launch_dwt_fwd_multi(kSrcRgbU8, 1, (const FwdLevelParams*)P(g, L_FWD0), M(g, L_FWD0), L[g][L_FWD0].total, L[g][L_FWD0].kind, st); }, "forward DWT") &&
+                   go(g, L_FWD0_COLOR, [&] { return launch_dwt_fwd_multi(kSrcRgbU8, 3, (const FwdLevelParams*)P(g, L_FWD0_COLOR), M(g, L_FWD0_COLOR), L[g][L_FWD0_COLOR].total, L[g][L_FWD0_COLOR].kind, st); }, "forward DWT");
         };
         auto fwdl = [&](int g, cudaStream_t st) {
             for (int k = L_FWD1; k <= L_FWD3; k++)
-                if (!go(g, k, [&] { return launch_dwt_fwd_multi(kSrcPlanes, (const FwdLevelParams*)P(g, k), M(g, k), L[g][k].total, L[g][k].kind, st); }, "forward DWT"))
+                if (!go(g, k, [&] { return launch_dwt_fwd_multi(kSrcPlanes, 1, (const FwdLevelParams*)P(g, k), M(g, k), L[g][k].total, L[g][k].kind, st); }, "forward DWT"))
                     return false;
             return true;
         };

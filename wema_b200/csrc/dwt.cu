@@ -3,11 +3,11 @@
 // pairs of columns per lane and a pair of rows at a time, both directions in
 // registers.
 //
-// Forward: RGB (converted on the way in; colour: the three channels of a pixel
-// together) or the previous level's LL in; LL and the three bands out, with
-// the temporal filter's step on each coefficient as it is written (batched
-// streams after their first frame).  Inverse: the bands are amplified as they
-// come in; planes out, or for colour at level 0 RGB.
+// Forward: RGB (converted on the way in, a channel at a time) or the previous
+// level's LL in; LL and the three bands out, with the temporal filter's step on
+// each coefficient as it is written (batched streams with FP32 state, after their
+// first frame).  Inverse: the bands are amplified as they come in; planes out, or
+// for colour at level 0 RGB.
 //
 // Sample and pair indices are 32-bit: the runtime caps frames at 2^28 pixels.
 // Arithmetic is the reference's: x = fma(left + right, c, x), scalings as
@@ -53,11 +53,11 @@ struct StateRing {
 };
 
 // What a sweep of channel z of a level uses of its parameters; what it rarely
-// uses stays in g.  F64: the biquad state and its update in FP64.  (A colour
-// frame's three channels are swept apart, each converting the pixels to its
-// own: the pixels are 3 of a channel's 34 bytes per pixel, and three channels'
-// rings and lifting state in one warp would leave one CTA per SM.)
-template <int MODE, bool H16, bool F64>
+// uses stays in g.  (A colour frame's three channels are swept apart, each
+// converting the pixels to its own: the pixels are 3 of a channel's 34 bytes per
+// pixel, and three channels' rings and lifting state in one warp would leave one
+// CTA per SM.)
+template <int MODE, bool H16>
 struct FwdSweep {
     const FwdLevelParams& g;
     int z, iw, ih, sw, sh, n, unit, vec_end;
@@ -212,7 +212,7 @@ __device__ __forceinline__ float pl_ldcg(const float* p, int i, bool h) {
 // filter reads the coefficient as stored (FP16-rounded in the planes_fp16
 // variant), so the deltas equal those of the separate filter kernel bit for bit.
 // tail: some coefficient of the row takes the scalar-tail form (uniform).
-template <bool H16, bool F64, class S>
+template <bool H16, class S>
 __device__ __forceinline__ void put_level(const S& p, int y, int g, bool second, bool tail,
                                           const float4 (*state)[32 * SQ], const float (&ll)[SQ], float (&v)[3][SQ]) {
     const int o = y * p.sw + g, lane = threadIdx.x & 31;
@@ -228,36 +228,24 @@ __device__ __forceinline__ void put_level(const S& p, int y, int g, bool second,
 #pragma unroll
             for (int k = 0; k < SQ; k++) v[b][k] = __half2float(__float2half_rn(v[b][k]));
         }
-        if constexpr (F64) {
+        float4 s[SQ];
 #pragma unroll
-            for (int k = 0; k < SQ; k++) {
-                if (k && !second) break;
-                double2* s2 = static_cast<double2*>(p.st) + 2 * (long long)(u + k);
-                double2 hp = __ldcs(s2), lp = __ldcs(s2 + 1);
-                v[b][k] = cascade64(p.c, hp, lp, v[b][k]);
-                __stcs(s2, hp);
-                __stcs(s2 + 1, lp);
-            }
+        for (int k = 0; k < SQ; k++) s[k] = state[b][SQ * lane + k];
+        if (!tail) {
+#pragma unroll
+            for (int k = 0; k < SQ; k++) v[b][k] = cascade(p.c, s[k], v[b][k], false);
         } else {
-            float4 s[SQ];
+            const long long u6 = p.g.iir_off6 + u;
 #pragma unroll
-            for (int k = 0; k < SQ; k++) s[k] = state[b][SQ * lane + k];
-            if (!tail) {
-#pragma unroll
-                for (int k = 0; k < SQ; k++) v[b][k] = cascade(p.c, s[k], v[b][k], false);
-            } else {
-                const long long u6 = p.g.iir_off6 + u;
-#pragma unroll
-                for (int k = 0; k < SQ; k++) v[b][k] = cascade(p.c, s[k], v[b][k], u6 + k >= p.g.iir_simd_end);
-            }
-            st_state2(static_cast<float4*>(p.st) + u, p.svec, second, s[0], s[1]);
+            for (int k = 0; k < SQ; k++) v[b][k] = cascade(p.c, s[k], v[b][k], u6 + k >= p.g.iir_simd_end);
         }
+        st_state2(static_cast<float4*>(p.st) + u, p.svec, second, s[0], s[1]);
         st_pair(p.dl, u, v[b], H16, cvec, second);
     }
 }
 
-template <int MODE, bool H16, bool F64, bool EDGE>
-__device__ __forceinline__ void fwd_sweep(const FwdSweep<MODE, H16, F64>& p, RowRing<MODE>& rows, StateRing* states,
+template <int MODE, bool H16, bool EDGE>
+__device__ __forceinline__ void fwd_sweep(const FwdSweep<MODE, H16>& p, RowRing<MODE>& rows, StateRing* states,
                                           const Strip<SQ>& s, int ya, int yb) {
     const int lane = threadIdx.x & 31;
     const int g = s.p0 + SQ * lane;
@@ -273,7 +261,7 @@ __device__ __forceinline__ void fwd_sweep(const FwdSweep<MODE, H16, F64>& p, Row
     const int j0 = ya - 2, j1 = yb + 2;
     auto issue = [&](int j, int slot) {
         if (j < j1) row_issue<MODE>(p, rows, slot, j, s.p0);
-        if (!F64 && p.st && j - 2 >= ya && j < j1) state_issue(p, *states, slot, j - 2, s);
+        if (p.st && j - 2 >= ya && j < j1) state_issue(p, *states, slot, j - 2, s);
         cp_commit();
     };
     __syncwarp();                            // the last segment's readers are done with the rings
@@ -336,7 +324,7 @@ __device__ __forceinline__ void fwd_sweep(const FwdSweep<MODE, H16, F64>& p, Row
             }
         }
         const bool tail = p.g.iir_off6 + 2 * p.n + (long long)y * p.sw + s.p0 + s.hi > p.g.iir_simd_end;
-        put_level<H16, F64>(p, y, g, second, tail, states->v[now], e, v);
+        put_level<H16>(p, y, g, second, tail, states->v[now], e, v);
     }
 }
 
@@ -347,15 +335,15 @@ __device__ __forceinline__ bool strip_edge(const Strip<SQ>& s, int w, int h, int
 }
 
 // units u0 .. u0 + n - 1 (p.unit pairs of rows each) of a CTA's group of strips
-template <int MODE, bool H16, bool F64>
+template <int MODE, bool H16>
 __device__ __forceinline__ void fwd_segment(const FwdLevelParams& g, int z, RowRing<MODE>& rows, StateRing* states,
                                             int group, int u0, int n) {
-    const FwdSweep<MODE, H16, F64> p(g, z);
+    const FwdSweep<MODE, H16> p(g, z);
     const Strip<SQ> s(group * SW_WARPS + (threadIdx.x >> 5), p.sw);
     if (s.hi <= s.lo) return;
     const int ya = u0 * p.unit, yb = min(ya + n * p.unit, p.sh);
-    if (strip_edge(s, p.iw, p.ih, p.sw)) fwd_sweep<MODE, H16, F64, true>(p, rows, states, s, ya, yb);
-    else fwd_sweep<MODE, H16, F64, false>(p, rows, states, s, ya, yb);
+    if (strip_edge(s, p.iw, p.ih, p.sw)) fwd_sweep<MODE, H16, true>(p, rows, states, s, ya, yb);
+    else fwd_sweep<MODE, H16, false>(p, rows, states, s, ya, yb);
 }
 
 // ----------------------------------------------------------------- inverse
@@ -585,10 +573,8 @@ __device__ __forceinline__ void inv_segment(const InvSweep<C, H16>& p, int group
 constexpr int fwd_res(int mode, bool rings) { return mode == kSrcRgbF32 ? 3 : rings ? 4 : 5; }
 constexpr int inv_res(int C) { return C == 3 ? 2 : 5; }
 
-// Storage types: FP32, or the precision variants' FP16 planes (1) and FP64
-// state (2).  One stream's kernel is compiled for its own; a batched launch
-// whose tasks agree takes that kernel too (KIND 0..3), one whose tasks differ
-// the kernel that holds them all (KIND -1).
+// Storage types: FP32, or the planes_fp16 variant's FP16 planes (H16): each launch's
+// kernel is compiled for its own.
 // f(first unit in the group, group, channel, units) for each segment of this CTA
 template <class F>
 __device__ __forceinline__ void each_segment(int units, int per, int groups, F f) {
@@ -603,27 +589,12 @@ __device__ __forceinline__ int groups_of(int pairs) {
     return (pairs + SW_WARPS * SW_LANES * SQ - 1) / (SW_WARPS * SW_LANES * SQ);
 }
 
-template <int MODE, int KIND>
-__device__ __forceinline__ void fwd_kind(const FwdLevelParams& g, int z, RowRing<MODE>& rows, StateRing* states,
-                                         int group, int row, int n) {
-    if constexpr (KIND >= 0) {
-        fwd_segment<MODE, (KIND & 1) != 0, (KIND & 2) != 0>(g, z, rows, states, group, row, n);
-    } else {
-        const bool f64 = g.iir_state[0] && g.iir_fp64;
-        if (g.h16 && f64) fwd_segment<MODE, true, true>(g, z, rows, states, group, row, n);
-        else if (g.h16) fwd_segment<MODE, true, false>(g, z, rows, states, group, row, n);
-        else if (f64) fwd_segment<MODE, false, true>(g, z, rows, states, group, row, n);
-        else fwd_segment<MODE, false, false>(g, z, rows, states, group, row, n);
-    }
-}
-int dwt_fwd_kind(const FwdLevelParams& p) { return (p.h16 ? 1 : 0) | (p.iir_state[0] && p.iir_fp64 ? 2 : 0); }
-
 template <int MODE, bool H16>
 __global__ void __launch_bounds__(SW_THREADS, fwd_res(MODE, false)) k_dwt_fwd(const __grid_constant__ FwdLevelParams g, int units) {
     __shared__ RowRing<MODE> rows[SW_WARPS];
     // (a plain session's filter is a launch of its own: no state here)
     each_segment(units, (g.sh + g.unit - 1) / g.unit, groups_of(g.sw), [&](int row, int group, int z, int n) {
-        fwd_kind<MODE, H16 ? 1 : 0>(g, z, rows[threadIdx.x >> 5], nullptr, group, row, n);
+        fwd_segment<MODE, H16>(g, z, rows[threadIdx.x >> 5], nullptr, group, row, n);
     });
 }
 template <int C, int OUT, bool H16>
@@ -666,9 +637,9 @@ __global__ void __cluster_dims__(TAIL_CTAS, 1, 1) __launch_bounds__(32 * TAIL_WA
 #pragma unroll 1
     for (int l = 0; l < t.count; l++) {
         if (l) cluster_barrier();
-        const FwdSweep<kSrcPlanes, H16, false> p(t.lv[l], blockIdx.y);
+        const FwdSweep<kSrcPlanes, H16> p(t.lv[l], blockIdx.y);
         tail_shares(p.sw, p.sh, [&](const Strip<SQ>& s, int ya, int yb) {
-            fwd_sweep<kSrcPlanes, H16, false, true>(p, rows[threadIdx.x >> 5], nullptr, s, ya, yb);
+            fwd_sweep<kSrcPlanes, H16, true>(p, rows[threadIdx.x >> 5], nullptr, s, ya, yb);
         });
     }
 }
@@ -696,23 +667,21 @@ __device__ __forceinline__ void each_task(const int* map, F f) {
         u.x += n;
     }
 }
-template <int MODE, int KIND>
+template <int MODE, bool H16>
 __global__ void __launch_bounds__(SW_THREADS, fwd_res(MODE, true))
     k_dwt_fwd_multi(const FwdLevelParams* __restrict__ ps, const int* __restrict__ map) {
     extern __shared__ __align__(16) unsigned char fwd_smem[];
     StateRing* const states = reinterpret_cast<StateRing*>(fwd_smem) + (threadIdx.x >> 5);
     RowRing<MODE>& rows = reinterpret_cast<RowRing<MODE>*>(fwd_smem + SW_WARPS * sizeof(StateRing))[threadIdx.x >> 5];
     each_task(map, [&](const TaskBlock& t, int n) {
-        fwd_kind<MODE, KIND>(ps[t.task], t.z, rows, states, t.y, t.x, n);
+        fwd_segment<MODE, H16>(ps[t.task], t.z, rows, states, t.y, t.x, n);
     });
 }
-template <int C, int OUT, int KIND>      // (KIND: FP16 planes or not, -1 both)
+template <int C, int OUT, bool H16>
 __global__ void __launch_bounds__(SW_THREADS, inv_res(C))
     k_dwt_inv_multi(const InvLevelParams* __restrict__ ps, const int* __restrict__ map) {
     each_task(map, [&](const TaskBlock& t, int n) {
-        const InvLevelParams& g = ps[t.task];
-        if (KIND > 0 || (KIND < 0 && g.h16)) inv_segment<C, OUT, KIND != 0>(InvSweep<C, KIND != 0>(g, t.z), t.y, t.x, n);
-        else inv_segment<C, OUT, false>(InvSweep<C, false>(g, t.z), t.y, t.x, n);
+        inv_segment<C, OUT, H16>(InvSweep<C, H16>(ps[t.task], t.z), t.y, t.x, n);
     });
 }
 
@@ -775,11 +744,13 @@ static unsigned sweep_grid(int& unit, int sw, int sh, int channels_z, int invers
     gy = (unsigned)sweep_groups(sw, SQ);
     return gx * gy * (unsigned)channels_z;
 }
-// a level's units (gx per group of strips, gy groups); sets p.unit
-unsigned dwt_fwd_grid(FwdLevelParams& p, int channels_z, unsigned& gx, unsigned& gy) {
+// a level's units (gx per group of strips, gy groups), and sets p.unit; or its tiles
+unsigned dwt_fwd_grid(FwdLevelParams& p, int channels_z, int form, unsigned& gx, unsigned& gy) {
+    if (form >= kDwtTiles) return tiles_grid(p.sw, p.sh, channels_z, gx, gy);
     return sweep_grid(p.unit, p.sw, p.sh, channels_z, 0, gx, gy);
 }
-unsigned dwt_inv_grid(InvLevelParams& p, int channels_z, unsigned& gx, unsigned& gy) {
+unsigned dwt_inv_grid(InvLevelParams& p, int channels_z, int form, unsigned& gx, unsigned& gy) {
+    if (form >= kDwtTiles) return tiles_grid(p.sw, p.sh, channels_z, gx, gy);
     return sweep_grid(p.unit, p.sw, p.sh, channels_z, 1, gx, gy);
 }
 
@@ -791,8 +762,7 @@ constexpr int ring_bytes() { return (int)(SW_WARPS * (sizeof(StateRing) + sizeof
 template <int MODE>
 static cudaError_t prepare_fwd() {
     cudaError_t e = cudaSuccess;
-    for (const void* k : {(const void*)k_dwt_fwd_multi<MODE, 0>, (const void*)k_dwt_fwd_multi<MODE, 1>,
-                          (const void*)k_dwt_fwd_multi<MODE, 2>, (const void*)k_dwt_fwd_multi<MODE, -1>}) {
+    for (const void* k : {(const void*)k_dwt_fwd_multi<MODE, false>, (const void*)k_dwt_fwd_multi<MODE, true>}) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, ring_bytes<MODE>());
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -800,41 +770,39 @@ static cudaError_t prepare_fwd() {
     return e;
 }
 cudaError_t dwt_prepare_device() {
-    const cudaError_t e = prepare_fwd<kSrcRgbU8>();
-    return e == cudaSuccess ? prepare_fwd<kSrcPlanes>() : e;
+    cudaError_t e = prepare_fwd<kSrcRgbU8>();
+    if (e == cudaSuccess) e = prepare_fwd<kSrcPlanes>();
+    return e == cudaSuccess ? tiles_prepare_device() : e;
 }
 
 template <int MODE>
-static void go_fwd_multi(int kind, const FwdLevelParams* ps, const int* map, int ctas, cudaStream_t st) {
-    switch (kind) {
-        case 0: k_dwt_fwd_multi<MODE, 0><<<ctas, SW_THREADS, ring_bytes<MODE>(), st>>>(ps, map); break;
-        case 1: k_dwt_fwd_multi<MODE, 1><<<ctas, SW_THREADS, ring_bytes<MODE>(), st>>>(ps, map); break;
-        case 2: k_dwt_fwd_multi<MODE, 2><<<ctas, SW_THREADS, ring_bytes<MODE>(), st>>>(ps, map); break;
-        default: k_dwt_fwd_multi<MODE, -1><<<ctas, SW_THREADS, ring_bytes<MODE>(), st>>>(ps, map); break;
-    }
+static void go_fwd_multi(bool h16, const FwdLevelParams* ps, const int* map, int ctas, cudaStream_t st) {
+    if (h16) k_dwt_fwd_multi<MODE, true><<<ctas, SW_THREADS, ring_bytes<MODE>(), st>>>(ps, map);
+    else k_dwt_fwd_multi<MODE, false><<<ctas, SW_THREADS, ring_bytes<MODE>(), st>>>(ps, map);
 }
-cudaError_t launch_dwt_fwd_multi(int mode, const FwdLevelParams* d_params, const int* d_map, unsigned blocks, int kind,
-                                 cudaStream_t st) {
+cudaError_t launch_dwt_fwd_multi(int mode, int channels, const FwdLevelParams* d_params, const int* d_map, unsigned blocks,
+                                 int form, cudaStream_t st) {
     if (blocks == 0) return cudaSuccess;
+    if (form >= kDwtTiles) return launch_tiles_fwd_multi(mode, channels, d_params, d_map, blocks, form == kDwtTiles16, st);
     const int n = ctas_for((int)blocks, 0, fwd_res(mode, true));
-    if (mode == kSrcPlanes) go_fwd_multi<kSrcPlanes>(kind, d_params, d_map, n, st);
-    else if (mode == kSrcRgbU8) go_fwd_multi<kSrcRgbU8>(kind, d_params, d_map, n, st);
+    if (mode == kSrcPlanes) go_fwd_multi<kSrcPlanes>(form == kDwtSweep16, d_params, d_map, n, st);
+    else if (mode == kSrcRgbU8) go_fwd_multi<kSrcRgbU8>(form == kDwtSweep16, d_params, d_map, n, st);
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
 
 template <int C, int OUT>
-static void go_inv_multi(int kind, const InvLevelParams* ps, const int* map, int ctas, cudaStream_t st) {
-    if (kind == 0) k_dwt_inv_multi<C, OUT, 0><<<ctas, SW_THREADS, 0, st>>>(ps, map);
-    else if (kind == 1) k_dwt_inv_multi<C, OUT, 1><<<ctas, SW_THREADS, 0, st>>>(ps, map);
-    else k_dwt_inv_multi<C, OUT, -1><<<ctas, SW_THREADS, 0, st>>>(ps, map);
+static void go_inv_multi(bool h16, const InvLevelParams* ps, const int* map, int ctas, cudaStream_t st) {
+    if (h16) k_dwt_inv_multi<C, OUT, true><<<ctas, SW_THREADS, 0, st>>>(ps, map);
+    else k_dwt_inv_multi<C, OUT, false><<<ctas, SW_THREADS, 0, st>>>(ps, map);
 }
 cudaError_t launch_dwt_inv_multi(int channels, int out_mode, const InvLevelParams* d_params,
-                                 const int* d_map, unsigned blocks, int kind, cudaStream_t st) {
+                                 const int* d_map, unsigned blocks, int form, cudaStream_t st) {
     if (blocks == 0) return cudaSuccess;
+    if (form >= kDwtTiles) return launch_tiles_inv_multi(channels, out_mode, d_params, d_map, blocks, st);
     const int n = ctas_for((int)blocks, 1, inv_res(channels));
-    if (out_mode == kOutRgb && channels == 3) go_inv_multi<3, kOutRgb>(kind, d_params, d_map, n, st);
-    else if (out_mode == kOutPlanes) go_inv_multi<1, kOutPlanes>(kind, d_params, d_map, n, st);
+    if (out_mode == kOutRgb && channels == 3) go_inv_multi<3, kOutRgb>(form == kDwtSweep16, d_params, d_map, n, st);
+    else if (out_mode == kOutPlanes) go_inv_multi<1, kOutPlanes>(form == kDwtSweep16, d_params, d_map, n, st);
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
@@ -849,7 +817,7 @@ cudaError_t launch_dwt_fwd(int mode, int channels, const FwdLevelParams& p0, cud
     if (channels != 1 && channels != 3) return cudaErrorInvalidValue;
     FwdLevelParams p = p0;
     unsigned gx, gy;
-    const int units = (int)dwt_fwd_grid(p, channels, gx, gy);
+    const int units = (int)dwt_fwd_grid(p, channels, kDwtSweep, gx, gy);
     if (mode == kSrcPlanes) go_fwd<kSrcPlanes>(p, units, st);
     else if (mode == kSrcRgbU8) go_fwd<kSrcRgbU8>(p, units, st);
     else if (mode == kSrcRgbF32) go_fwd<kSrcRgbF32>(p, units, st);
@@ -866,7 +834,7 @@ static void go_inv(const InvLevelParams& p, int units, cudaStream_t st) {
 cudaError_t launch_dwt_inv(int channels, int out_mode, const InvLevelParams& p0, cudaStream_t st) {
     InvLevelParams p = p0;
     unsigned gx, gy;
-    const int units = (int)dwt_inv_grid(p, out_mode == kOutPlanes ? channels : 1, gx, gy);
+    const int units = (int)dwt_inv_grid(p, out_mode == kOutPlanes ? channels : 1, kDwtSweep, gx, gy);
     if (out_mode == kOutPlanes && (channels == 1 || channels == 3)) go_inv<1, kOutPlanes>(p, units, st);
     else if (out_mode == kOutRgb && channels == 3) go_inv<3, kOutRgb>(p, units, st);
     else return cudaErrorInvalidValue;
@@ -994,7 +962,7 @@ cudaError_t dwt_autotune(int dev, float fwd_ms[9], float inv_ms[9], int* fwd_bes
         for (int v = 0; v < kDwtVariants; v++) {
             dwt_set_variant(dev, inv, v);
             unsigned gx, gy;
-            const unsigned units = inv ? dwt_inv_grid(ip, 1, gx, gy) : dwt_fwd_grid(fp, 1, gx, gy);
+            const unsigned units = inv ? dwt_inv_grid(ip, 1, kDwtSweep, gx, gy) : dwt_fwd_grid(fp, 1, kDwtSweep, gx, gy);
             const int m[5] = {1, 0, (int)units, (int)gx, (int)gy};
             if ((e = cudaMemcpy(map, m, sizeof m, cudaMemcpyHostToDevice)) != cudaSuccess) return done(e);
             e = inv ? cudaMemcpy(dpi, &ip, sizeof ip, cudaMemcpyHostToDevice)
@@ -1002,8 +970,8 @@ cudaError_t dwt_autotune(int dev, float fwd_ms[9], float inv_ms[9], int* fwd_bes
             if (e != cudaSuccess) return done(e);
             for (int rep = 0; rep < 6; rep++) {
                 if (rep == 1 && (e = cudaEventRecord(e0, st)) != cudaSuccess) return done(e);
-                e = inv ? launch_dwt_inv_multi(1, kOutPlanes, (const InvLevelParams*)dpi, map, units, 0, st)
-                        : launch_dwt_fwd_multi(kSrcRgbU8, (const FwdLevelParams*)dp, map, units, 0, st);
+                e = inv ? launch_dwt_inv_multi(1, kOutPlanes, (const InvLevelParams*)dpi, map, units, kDwtSweep, st)
+                        : launch_dwt_fwd_multi(kSrcRgbU8, 1, (const FwdLevelParams*)dp, map, units, kDwtSweep, st);
                 if (e != cudaSuccess) return done(e);
             }
             if ((e = cudaEventRecord(e1, st)) != cudaSuccess) return done(e);

@@ -162,14 +162,25 @@ cudaError_t launch_window(const WindowParams& wp, int channels, cudaStream_t st)
 // ---- batched launches: one launch of a kernel over many streams --------------
 // Every launch takes a device array of per-task parameters and a task map
 // (multi.cuh); `blocks` is the sum of the tasks' grids.
-unsigned dwt_fwd_grid(FwdLevelParams& p, int channels_z, unsigned& gx, unsigned& gy);
-unsigned dwt_inv_grid(InvLevelParams& p, int channels_z, unsigned& gx, unsigned& gy);
-// kind: the tasks' common dwt_fwd_kind (inverse: h16), or -1 when they differ
-int dwt_fwd_kind(const FwdLevelParams& p);
-cudaError_t launch_dwt_fwd_multi(int mode, const FwdLevelParams* d_params, const int* d_map, unsigned blocks, int kind,
-                                 cudaStream_t st);
+// How a batched DWT launch goes: by sweeps (dwt.cu), FP32 planes or FP16 ones; or by
+// tiles (dwt_tiles.cu), with FP16 planes among its tasks or without.  The sweeps'
+// map counts units, and their level 0 takes luma and colour streams together (a
+// channel at a time); the tiles' counts tiles, a colour stream's level 0 in a launch
+// of its own.
+enum { kDwtSweep = 0, kDwtSweep16 = 1, kDwtTiles = 2, kDwtTiles16 = 3 };
+unsigned dwt_fwd_grid(FwdLevelParams& p, int channels_z, int form, unsigned& gx, unsigned& gy);
+unsigned dwt_inv_grid(InvLevelParams& p, int channels_z, int form, unsigned& gx, unsigned& gy);
+cudaError_t launch_dwt_fwd_multi(int mode, int channels, const FwdLevelParams* d_params, const int* d_map, unsigned blocks,
+                                 int form, cudaStream_t st);
 cudaError_t launch_dwt_inv_multi(int channels, int out_mode, const InvLevelParams* d_params,
-                                 const int* d_map, unsigned blocks, int kind, cudaStream_t st);
+                                 const int* d_map, unsigned blocks, int form, cudaStream_t st);
+// the tiles (dwt_tiles.cu), behind the functions above
+cudaError_t tiles_prepare_device();
+unsigned tiles_grid(int sw, int sh, int channels_z, unsigned& gx, unsigned& gy);
+cudaError_t launch_tiles_fwd_multi(int mode, int channels, const FwdLevelParams* d_params, const int* d_map,
+                                   unsigned blocks, bool any16, cudaStream_t st);
+cudaError_t launch_tiles_inv_multi(int channels, int out_mode, const InvLevelParams* d_params, const int* d_map,
+                                   unsigned blocks, cudaStream_t st);
 size_t thr_args_bytes();
 // grids[stage] = {x, y} for stage 0 partials, 1 prefix, 2 monoids, 3 walk
 cudaError_t thr_args_fill(void* dst, const PyrView* views, int nch, const ThrScratch* scratch,
