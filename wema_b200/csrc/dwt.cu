@@ -339,11 +339,12 @@ template <int MODE, bool H16>
 __device__ __forceinline__ void fwd_segment(const FwdLevelParams& g, int z, RowRing<MODE>& rows, StateRing* states,
                                             int group, int u0, int n) {
     const FwdSweep<MODE, H16> p(g, z);
-    const Strip<SQ> s(group * SW_WARPS + (threadIdx.x >> 5), p.sw);
-    if (s.hi <= s.lo) return;
-    const int ya = u0 * p.unit, yb = min(ya + n * p.unit, p.sh);
-    if (strip_edge(s, p.iw, p.ih, p.sw)) fwd_sweep<MODE, H16, true>(p, rows, states, s, ya, yb);
-    else fwd_sweep<MODE, H16, false>(p, rows, states, s, ya, yb);
+    const int across = sweep_across(p.sw, SQ);
+    const WarpRows r(across, u0 * p.unit, min((u0 + n) * p.unit, p.sh));
+    const Strip<SQ> s(group * across + r.strip, p.sw);
+    if (s.hi <= s.lo || r.yb <= r.ya) return;
+    if (strip_edge(s, p.iw, p.ih, p.sw)) fwd_sweep<MODE, H16, true>(p, rows, states, s, r.ya, r.yb);
+    else fwd_sweep<MODE, H16, false>(p, rows, states, s, r.ya, r.yb);
 }
 
 // ----------------------------------------------------------------- inverse
@@ -554,11 +555,12 @@ __device__ __forceinline__ void inv_sweep(const InvSweep<C, H16>& p, const Strip
 
 template <int C, int OUT, bool H16>
 __device__ __forceinline__ void inv_segment(const InvSweep<C, H16>& p, int group, int u0, int n) {
-    const Strip<SQ> s(group * SW_WARPS + (threadIdx.x >> 5), p.sw);
-    if (s.hi <= s.lo) return;
-    const int ya = u0 * p.unit, yb = min(ya + n * p.unit, p.sh);
-    if (strip_edge(s, p.ow, p.oh, p.sw)) inv_sweep<C, OUT, H16, true>(p, s, ya, yb);
-    else inv_sweep<C, OUT, H16, false>(p, s, ya, yb);
+    const int across = sweep_across(p.sw, SQ);
+    const WarpRows r(across, u0 * p.unit, min((u0 + n) * p.unit, p.sh));
+    const Strip<SQ> s(group * across + r.strip, p.sw);
+    if (s.hi <= s.lo || r.yb <= r.ya) return;
+    if (strip_edge(s, p.ow, p.oh, p.sw)) inv_sweep<C, OUT, H16, true>(p, s, r.ya, r.yb);
+    else inv_sweep<C, OUT, H16, false>(p, s, r.ya, r.yb);
 }
 
 // ------------------------------------------------------------- wrappers
@@ -585,21 +587,18 @@ __device__ __forceinline__ void each_segment(int units, int per, int groups, F f
         u.x += n;
     }
 }
-__device__ __forceinline__ int groups_of(int pairs) {
-    return (pairs + SW_WARPS * SW_LANES * SQ - 1) / (SW_WARPS * SW_LANES * SQ);
-}
 
 template <int MODE, bool H16>
 __global__ void __launch_bounds__(SW_THREADS, fwd_res(MODE, false)) k_dwt_fwd(const __grid_constant__ FwdLevelParams g, int units) {
     __shared__ RowRing<MODE> rows[SW_WARPS];
     // (a plain session's filter is a launch of its own: no state here)
-    each_segment(units, (g.sh + g.unit - 1) / g.unit, groups_of(g.sw), [&](int row, int group, int z, int n) {
+    each_segment(units, (g.sh + g.unit - 1) / g.unit, sweep_groups(g.sw, SQ), [&](int row, int group, int z, int n) {
         fwd_segment<MODE, H16>(g, z, rows[threadIdx.x >> 5], nullptr, group, row, n);
     });
 }
 template <int C, int OUT, bool H16>
 __global__ void __launch_bounds__(SW_THREADS, inv_res(C)) k_dwt_inv(const __grid_constant__ InvLevelParams g, int units) {
-    each_segment(units, (g.sh + g.unit - 1) / g.unit, groups_of(g.sw), [&](int row, int group, int z, int n) {
+    each_segment(units, (g.sh + g.unit - 1) / g.unit, sweep_groups(g.sw, SQ), [&](int row, int group, int z, int n) {
         inv_segment<C, OUT, H16>(InvSweep<C, H16>(g, z), group, row, n);
     });
 }
@@ -740,6 +739,7 @@ static int ctas_for(int units, int inverse, int most) {
 static unsigned sweep_grid(int& unit, int sw, int sh, int channels_z, int inverse, unsigned& gx, unsigned& gy) {
     int res;
     dwt_variant_shape(dwt_variant(dwt_dev_now(), inverse), &res, &unit);
+    unit *= SW_WARPS / sweep_across(sw, SQ);          // (a warp's rows stay the setting's)
     gx = (unsigned)((sh + unit - 1) / unit);
     gy = (unsigned)sweep_groups(sw, SQ);
     return gx * gy * (unsigned)channels_z;

@@ -28,9 +28,27 @@ constexpr int SW_THREADS = 32 * SW_WARPS;
 constexpr int SW_LANES = 30;             // lanes of a strip that write
 constexpr unsigned SW_FULL = 0xffffffffu;
 
-// a CTA's warps take neighbouring strips over the same rows: the samples two
-// strips share then come from the first-level cache
-inline int sweep_groups(int pairs, int q) { return (pairs + SW_WARPS * SW_LANES * q - 1) / (SW_WARPS * SW_LANES * q); }
+// A CTA's warps take neighbouring strips over the same rows (the samples two
+// strips share then come from the first-level cache) where a level has three strips
+// or more; of one or two, the warps take a part of the rows each (with two or
+// three of them idle, eight 64x8192 streams in colour took 730 us a tick, so 354).
+inline __host__ __device__ int sweep_across(int pairs, int q) {   // strips of a CTA side by side: 1, 2 or 4
+    return pairs <= SW_LANES * q ? 1 : pairs <= 2 * SW_LANES * q ? 2 : SW_WARPS;
+}
+inline __host__ __device__ int sweep_groups(int pairs, int q) {
+    const int most = sweep_across(pairs, q) * SW_LANES * q;
+    return (pairs + most - 1) / most;
+}
+// this warp's part of rows ya .. yb - 1 that its CTA takes
+struct WarpRows {
+    int strip, ya, yb;                   // (of the CTA's strips, of the rows)
+    __device__ __forceinline__ WarpRows(int across, int a, int b) {
+        const int w = threadIdx.x >> 5, down = SW_WARPS / across, r = w / across;
+        strip = w % across;
+        ya = a + (b - a) * r / down;
+        yb = a + (b - a) * (r + 1) / down;
+    }
+};
 
 // strip s of a level of `sw` pairs: its first pair, and the range of its pairs
 // (from the first one) that it writes
