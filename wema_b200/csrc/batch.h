@@ -60,6 +60,7 @@ struct Launch {
     size_t params_off = 0, map_off = 0;   // device offsets in the tick's table
     int kind = -2;                        // the tasks' common form (transforms: kDwt..., guided transfer: rows),
                                           // -1 when they differ, -2 none
+    bool narrow = false;                  // transforms: some task's level is at most two strips wide
     void reset(size_t e) {
         elem = e;
         params.clear();
@@ -68,6 +69,7 @@ struct Launch {
         nblk.clear();
         total = 0;
         kind = -2;
+        narrow = false;
     }
     void add(const void* p, unsigned x, unsigned y, unsigned blocks) {
         if (blocks == 0) return;
@@ -563,6 +565,7 @@ public:
                 const unsigned b = dwt_fwd_grid(p, apart ? 1 : nch, ff, gx, gy);
                 lf.add(&p, gx, gy, b);
                 lf.merge(ff);
+                lf.narrow |= dwt_narrow(p.sw);
             }
             // ---- threshold
             PyrView views[3];
@@ -626,6 +629,7 @@ public:
                 const unsigned b = dwt_inv_grid(iq, l == 0 && nch == 3 ? 1 : nch, fi, gx, gy);
                 li.add(&iq, gx, gy, b);
                 li.merge(fi);
+                li.narrow |= dwt_narrow(iq.sw);
             }
             if (nch == 1) {
                 TransferParams tp{};
@@ -689,12 +693,12 @@ public:
 
         // the stages of one group on one stream
         auto fwd0 = [&](int g, cudaStream_t st) {
-            return go(g, L_FWD0, [&] { return launch_dwt_fwd_multi(kSrcRgbU8, 1, (const FwdLevelParams*)P(g, L_FWD0), M(g, L_FWD0), L[g][L_FWD0].total, L[g][L_FWD0].kind, st); }, "forward DWT") &&
-                   go(g, L_FWD0_COLOR, [&] { return launch_dwt_fwd_multi(kSrcRgbU8, 3, (const FwdLevelParams*)P(g, L_FWD0_COLOR), M(g, L_FWD0_COLOR), L[g][L_FWD0_COLOR].total, L[g][L_FWD0_COLOR].kind, st); }, "forward DWT");
+            return go(g, L_FWD0, [&] { return launch_dwt_fwd_multi(kSrcRgbU8, 1, (const FwdLevelParams*)P(g, L_FWD0), M(g, L_FWD0), L[g][L_FWD0].total, L[g][L_FWD0].kind, L[g][L_FWD0].narrow, st); }, "forward DWT") &&
+                   go(g, L_FWD0_COLOR, [&] { return launch_dwt_fwd_multi(kSrcRgbU8, 3, (const FwdLevelParams*)P(g, L_FWD0_COLOR), M(g, L_FWD0_COLOR), L[g][L_FWD0_COLOR].total, L[g][L_FWD0_COLOR].kind, L[g][L_FWD0_COLOR].narrow, st); }, "forward DWT");
         };
         auto fwdl = [&](int g, cudaStream_t st) {
             for (int k = L_FWD1; k <= L_FWD3; k++)
-                if (!go(g, k, [&] { return launch_dwt_fwd_multi(kSrcPlanes, 1, (const FwdLevelParams*)P(g, k), M(g, k), L[g][k].total, L[g][k].kind, st); }, "forward DWT"))
+                if (!go(g, k, [&] { return launch_dwt_fwd_multi(kSrcPlanes, 1, (const FwdLevelParams*)P(g, k), M(g, k), L[g][k].total, L[g][k].kind, L[g][k].narrow, st); }, "forward DWT"))
                     return false;
             return true;
         };
@@ -720,13 +724,13 @@ public:
         };
         auto invl = [&](int g, cudaStream_t st) {
             for (int k = L_INV3; k <= L_INV1; k++)
-                if (!go(g, k, [&] { return launch_dwt_inv_multi(1, kOutPlanes, (const InvLevelParams*)P(g, k), M(g, k), L[g][k].total, L[g][k].kind, st); }, "inverse DWT"))
+                if (!go(g, k, [&] { return launch_dwt_inv_multi(1, kOutPlanes, (const InvLevelParams*)P(g, k), M(g, k), L[g][k].total, L[g][k].kind, L[g][k].narrow, st); }, "inverse DWT"))
                     return false;
             return true;
         };
         auto inv0 = [&](int g, cudaStream_t st) {
-            return go(g, L_INV0_LUMA, [&] { return launch_dwt_inv_multi(1, kOutPlanes, (const InvLevelParams*)P(g, L_INV0_LUMA), M(g, L_INV0_LUMA), L[g][L_INV0_LUMA].total, L[g][L_INV0_LUMA].kind, st); }, "inverse DWT") &&
-                   go(g, L_INV0_COLOR, [&] { return launch_dwt_inv_multi(3, kOutRgb, (const InvLevelParams*)P(g, L_INV0_COLOR), M(g, L_INV0_COLOR), L[g][L_INV0_COLOR].total, L[g][L_INV0_COLOR].kind, st); }, "inverse DWT");
+            return go(g, L_INV0_LUMA, [&] { return launch_dwt_inv_multi(1, kOutPlanes, (const InvLevelParams*)P(g, L_INV0_LUMA), M(g, L_INV0_LUMA), L[g][L_INV0_LUMA].total, L[g][L_INV0_LUMA].kind, L[g][L_INV0_LUMA].narrow, st); }, "inverse DWT") &&
+                   go(g, L_INV0_COLOR, [&] { return launch_dwt_inv_multi(3, kOutRgb, (const InvLevelParams*)P(g, L_INV0_COLOR), M(g, L_INV0_COLOR), L[g][L_INV0_COLOR].total, L[g][L_INV0_COLOR].kind, L[g][L_INV0_COLOR].narrow, st); }, "inverse DWT");
         };
         auto xfer = [&](int g, cudaStream_t st) {
             return go(g, L_XFER_GUIDED, [&] { return launch_transfer_multi(1, (const TransferParams*)P(g, L_XFER_GUIDED), M(g, L_XFER_GUIDED), L[g][L_XFER_GUIDED].total, L[g][L_XFER_GUIDED].kind, st); }, "luma transfer") &&
@@ -787,7 +791,7 @@ public:
                     sig.push_back(l.total);
                     sig.push_back((long long)l.params_off);
                     sig.push_back((long long)l.map_off);
-                    sig.push_back(l.kind);
+                    sig.push_back(2 * l.kind + l.narrow);
                 }
             if (sig != t.sig) {
                 drop_graphs(t);

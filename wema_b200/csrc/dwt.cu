@@ -60,7 +60,7 @@ struct StateRing {
 template <int MODE, bool H16>
 struct FwdSweep {
     const FwdLevelParams& g;
-    int z, iw, ih, sw, sh, n, unit, vec_end;
+    int z, iw, ih, sw, sh, n, vec_end;
     int inner;                           // rows whose copies may be whole pieces (row_copy.h)
     const void* src;                     // RGB24, float RGB, or the channel's plane
     float *coef, *ll, *dl;
@@ -72,7 +72,7 @@ struct FwdSweep {
         return z == 0 ? a[0] : z == 1 ? a[1] : a[2];
     }
     __device__ __forceinline__ FwdSweep(const FwdLevelParams& g_, int z_)
-        : g(g_), z(z_), iw(g.iw), ih(g.ih), sw(g.sw), sh(g.sh), n((int)g.n), unit(g.unit), vec_end((int)g.vec_end) {
+        : g(g_), z(z_), iw(g.iw), ih(g.ih), sw(g.sw), sh(g.sh), n((int)g.n), vec_end((int)g.vec_end) {
         inner = inner_rows(ih, RowRing<MODE>::PX * iw);
         coef = pick(g.coef);
         ll = pick(g.ll_out);
@@ -334,15 +334,17 @@ __device__ __forceinline__ bool strip_edge(const Strip<SQ>& s, int w, int h, int
     return (w % (2 * SQ) != 0 && s.p0 + 32 * SQ >= pairs) || w < 2 || h < 2;
 }
 
-// units u0 .. u0 + n - 1 (p.unit pairs of rows each) of a CTA's group of strips
-template <int MODE, bool H16>
+// units u0 .. u0 + n - 1 (g.unit pairs of rows each) of a CTA's group of strips.
+// NARROW: the level may be one or two strips wide, whose rows the warps share; a
+// form of its own, as rows that differ from warp to warp make the wide levels'
+// sweeps 5 to 8% longer.
+template <int MODE, bool H16, bool NARROW>
 __device__ __forceinline__ void fwd_segment(const FwdLevelParams& g, int z, RowRing<MODE>& rows, StateRing* states,
                                             int group, int u0, int n) {
     const FwdSweep<MODE, H16> p(g, z);
-    const int across = sweep_across(p.sw, SQ);
-    const WarpRows r(across, u0 * p.unit, min((u0 + n) * p.unit, p.sh));
-    const Strip<SQ> s(group * across + r.strip, p.sw);
-    if (s.hi <= s.lo || r.yb <= r.ya) return;
+    const WarpRows<NARROW> r(group, sweep_across(p.sw, SQ), u0 * g.unit, min((u0 + n) * g.unit, p.sh));
+    const Strip<SQ> s(r.strip, p.sw);
+    if (s.hi <= s.lo || (NARROW && r.yb <= r.ya)) return;
     if (strip_edge(s, p.iw, p.ih, p.sw)) fwd_sweep<MODE, H16, true>(p, rows, states, s, r.ya, r.yb);
     else fwd_sweep<MODE, H16, false>(p, rows, states, s, r.ya, r.yb);
 }
@@ -352,7 +354,7 @@ __device__ __forceinline__ void fwd_segment(const FwdLevelParams& g, int z, RowR
 // OUT: kOutPlanes (one channel) or kOutRgb (three)
 template <int C, bool H16>
 struct InvSweep {
-    int ow, oh, sw, sh, n, unit;
+    int ow, oh, sw, sh, n;
     const float *ll[C], *coef[C], *delta[C];
     float* out[C];
     float thr[C], al[C];
@@ -360,7 +362,7 @@ struct InvSweep {
     float* f32;
     bool out16, vec, ovec, wvec;         // inputs, output planes, output bytes start at vectors
     __device__ __forceinline__ InvSweep(const InvLevelParams& g, int z)
-        : ow(g.ow), oh(g.oh), sw(g.sw), sh(g.sh), n((int)g.n), unit(g.unit), u8(g.out_u8), f32(g.out_f32) {
+        : ow(g.ow), oh(g.oh), sw(g.sw), sh(g.sh), n((int)g.n), u8(g.out_u8), f32(g.out_f32) {
         uintptr_t in = 0, planes = 0;
 #pragma unroll
         for (int k = 0; k < C; k++) {
@@ -553,12 +555,12 @@ __device__ __forceinline__ void inv_sweep(const InvSweep<C, H16>& p, const Strip
     }
 }
 
-template <int C, int OUT, bool H16>
-__device__ __forceinline__ void inv_segment(const InvSweep<C, H16>& p, int group, int u0, int n) {
-    const int across = sweep_across(p.sw, SQ);
-    const WarpRows r(across, u0 * p.unit, min((u0 + n) * p.unit, p.sh));
-    const Strip<SQ> s(group * across + r.strip, p.sw);
-    if (s.hi <= s.lo || r.yb <= r.ya) return;
+template <int C, int OUT, bool H16, bool NARROW>
+__device__ __forceinline__ void inv_segment(const InvLevelParams& g, int z, int group, int u0, int n) {
+    const InvSweep<C, H16> p(g, z);
+    const WarpRows<NARROW> r(group, sweep_across(p.sw, SQ), u0 * g.unit, min((u0 + n) * g.unit, p.sh));
+    const Strip<SQ> s(r.strip, p.sw);
+    if (s.hi <= s.lo || (NARROW && r.yb <= r.ya)) return;
     if (strip_edge(s, p.ow, p.oh, p.sw)) inv_sweep<C, OUT, H16, true>(p, s, r.ya, r.yb);
     else inv_sweep<C, OUT, H16, false>(p, s, r.ya, r.yb);
 }
@@ -593,13 +595,13 @@ __global__ void __launch_bounds__(SW_THREADS, fwd_res(MODE, false)) k_dwt_fwd(co
     __shared__ RowRing<MODE> rows[SW_WARPS];
     // (a plain session's filter is a launch of its own: no state here)
     each_segment(units, (g.sh + g.unit - 1) / g.unit, sweep_groups(g.sw, SQ), [&](int row, int group, int z, int n) {
-        fwd_segment<MODE, H16>(g, z, rows[threadIdx.x >> 5], nullptr, group, row, n);
+        fwd_segment<MODE, H16, false>(g, z, rows[threadIdx.x >> 5], nullptr, group, row, n);
     });
 }
 template <int C, int OUT, bool H16>
 __global__ void __launch_bounds__(SW_THREADS, inv_res(C)) k_dwt_inv(const __grid_constant__ InvLevelParams g, int units) {
     each_segment(units, (g.sh + g.unit - 1) / g.unit, sweep_groups(g.sw, SQ), [&](int row, int group, int z, int n) {
-        inv_segment<C, OUT, H16>(InvSweep<C, H16>(g, z), group, row, n);
+        inv_segment<C, OUT, H16, false>(g, z, group, row, n);
     });
 }
 
@@ -666,21 +668,21 @@ __device__ __forceinline__ void each_task(const int* map, F f) {
         u.x += n;
     }
 }
-template <int MODE, bool H16>
+template <int MODE, bool H16, bool NARROW>
 __global__ void __launch_bounds__(SW_THREADS, fwd_res(MODE, true))
     k_dwt_fwd_multi(const FwdLevelParams* __restrict__ ps, const int* __restrict__ map) {
     extern __shared__ __align__(16) unsigned char fwd_smem[];
     StateRing* const states = reinterpret_cast<StateRing*>(fwd_smem) + (threadIdx.x >> 5);
     RowRing<MODE>& rows = reinterpret_cast<RowRing<MODE>*>(fwd_smem + SW_WARPS * sizeof(StateRing))[threadIdx.x >> 5];
     each_task(map, [&](const TaskBlock& t, int n) {
-        fwd_segment<MODE, H16>(ps[t.task], t.z, rows, states, t.y, t.x, n);
+        fwd_segment<MODE, H16, NARROW>(ps[t.task], t.z, rows, states, t.y, t.x, n);
     });
 }
-template <int C, int OUT, bool H16>
+template <int C, int OUT, bool H16, bool NARROW>
 __global__ void __launch_bounds__(SW_THREADS, inv_res(C))
     k_dwt_inv_multi(const InvLevelParams* __restrict__ ps, const int* __restrict__ map) {
     each_task(map, [&](const TaskBlock& t, int n) {
-        inv_segment<C, OUT, H16>(InvSweep<C, H16>(ps[t.task], t.z), t.y, t.x, n);
+        inv_segment<C, OUT, H16, NARROW>(ps[t.task], t.z, t.y, t.x, n);
     });
 }
 
@@ -736,22 +738,23 @@ static int ctas_for(int units, int inverse, int most) {
 }
 
 // ----------------------------------------------------------------- launch
-static unsigned sweep_grid(int& unit, int sw, int sh, int channels_z, int inverse, unsigned& gx, unsigned& gy) {
+static unsigned sweep_grid(int& unit, int sw, int sh, int channels_z, int inverse, bool narrow, unsigned& gx, unsigned& gy) {
     int res;
     dwt_variant_shape(dwt_variant(dwt_dev_now(), inverse), &res, &unit);
-    unit *= SW_WARPS / sweep_across(sw, SQ);          // (a warp's rows stay the setting's)
+    if (narrow) unit *= SW_WARPS / sweep_across(sw, SQ);   // (a warp's rows stay the setting's)
     gx = (unsigned)((sh + unit - 1) / unit);
     gy = (unsigned)sweep_groups(sw, SQ);
     return gx * gy * (unsigned)channels_z;
 }
-// a level's units (gx per group of strips, gy groups), and sets p.unit; or its tiles
+bool dwt_narrow(int sw) { return sweep_across(sw, SQ) < SW_WARPS; }
+// a task's units (gx per group of strips, gy groups), and sets p.unit; or its tiles
 unsigned dwt_fwd_grid(FwdLevelParams& p, int channels_z, int form, unsigned& gx, unsigned& gy) {
     if (form >= kDwtTiles) return tiles_grid(p.sw, p.sh, channels_z, gx, gy);
-    return sweep_grid(p.unit, p.sw, p.sh, channels_z, 0, gx, gy);
+    return sweep_grid(p.unit, p.sw, p.sh, channels_z, 0, true, gx, gy);
 }
 unsigned dwt_inv_grid(InvLevelParams& p, int channels_z, int form, unsigned& gx, unsigned& gy) {
     if (form >= kDwtTiles) return tiles_grid(p.sw, p.sh, channels_z, gx, gy);
-    return sweep_grid(p.unit, p.sw, p.sh, channels_z, 1, gx, gy);
+    return sweep_grid(p.unit, p.sw, p.sh, channels_z, 1, true, gx, gy);
 }
 
 template <int MODE>
@@ -762,7 +765,8 @@ constexpr int ring_bytes() { return (int)(SW_WARPS * (sizeof(StateRing) + sizeof
 template <int MODE>
 static cudaError_t prepare_fwd() {
     cudaError_t e = cudaSuccess;
-    for (const void* k : {(const void*)k_dwt_fwd_multi<MODE, false>, (const void*)k_dwt_fwd_multi<MODE, true>}) {
+    for (const void* k : {(const void*)k_dwt_fwd_multi<MODE, false, false>, (const void*)k_dwt_fwd_multi<MODE, true, false>,
+                          (const void*)k_dwt_fwd_multi<MODE, false, true>, (const void*)k_dwt_fwd_multi<MODE, true, true>}) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, ring_bytes<MODE>());
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
@@ -775,34 +779,40 @@ cudaError_t dwt_prepare_device() {
     return e == cudaSuccess ? tiles_prepare_device() : e;
 }
 
-template <int MODE>
+template <int MODE, bool NARROW>
 static void go_fwd_multi(bool h16, const FwdLevelParams* ps, const int* map, int ctas, cudaStream_t st) {
-    if (h16) k_dwt_fwd_multi<MODE, true><<<ctas, SW_THREADS, ring_bytes<MODE>(), st>>>(ps, map);
-    else k_dwt_fwd_multi<MODE, false><<<ctas, SW_THREADS, ring_bytes<MODE>(), st>>>(ps, map);
+    if (h16) k_dwt_fwd_multi<MODE, true, NARROW><<<ctas, SW_THREADS, ring_bytes<MODE>(), st>>>(ps, map);
+    else k_dwt_fwd_multi<MODE, false, NARROW><<<ctas, SW_THREADS, ring_bytes<MODE>(), st>>>(ps, map);
 }
 cudaError_t launch_dwt_fwd_multi(int mode, int channels, const FwdLevelParams* d_params, const int* d_map, unsigned blocks,
-                                 int form, cudaStream_t st) {
+                                 int form, bool narrow, cudaStream_t st) {
     if (blocks == 0) return cudaSuccess;
     if (form >= kDwtTiles) return launch_tiles_fwd_multi(mode, channels, d_params, d_map, blocks, form == kDwtTiles16, st);
     const int n = ctas_for((int)blocks, 0, fwd_res(mode, true));
-    if (mode == kSrcPlanes) go_fwd_multi<kSrcPlanes>(form == kDwtSweep16, d_params, d_map, n, st);
-    else if (mode == kSrcRgbU8) go_fwd_multi<kSrcRgbU8>(form == kDwtSweep16, d_params, d_map, n, st);
+    const bool h16 = form == kDwtSweep16;
+    if (mode == kSrcPlanes && narrow) go_fwd_multi<kSrcPlanes, true>(h16, d_params, d_map, n, st);
+    else if (mode == kSrcPlanes) go_fwd_multi<kSrcPlanes, false>(h16, d_params, d_map, n, st);
+    else if (mode == kSrcRgbU8 && narrow) go_fwd_multi<kSrcRgbU8, true>(h16, d_params, d_map, n, st);
+    else if (mode == kSrcRgbU8) go_fwd_multi<kSrcRgbU8, false>(h16, d_params, d_map, n, st);
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
 
-template <int C, int OUT>
+template <int C, int OUT, bool NARROW>
 static void go_inv_multi(bool h16, const InvLevelParams* ps, const int* map, int ctas, cudaStream_t st) {
-    if (h16) k_dwt_inv_multi<C, OUT, true><<<ctas, SW_THREADS, 0, st>>>(ps, map);
-    else k_dwt_inv_multi<C, OUT, false><<<ctas, SW_THREADS, 0, st>>>(ps, map);
+    if (h16) k_dwt_inv_multi<C, OUT, true, NARROW><<<ctas, SW_THREADS, 0, st>>>(ps, map);
+    else k_dwt_inv_multi<C, OUT, false, NARROW><<<ctas, SW_THREADS, 0, st>>>(ps, map);
 }
 cudaError_t launch_dwt_inv_multi(int channels, int out_mode, const InvLevelParams* d_params,
-                                 const int* d_map, unsigned blocks, int form, cudaStream_t st) {
+                                 const int* d_map, unsigned blocks, int form, bool narrow, cudaStream_t st) {
     if (blocks == 0) return cudaSuccess;
     if (form >= kDwtTiles) return launch_tiles_inv_multi(channels, out_mode, d_params, d_map, blocks, st);
     const int n = ctas_for((int)blocks, 1, inv_res(channels));
-    if (out_mode == kOutRgb && channels == 3) go_inv_multi<3, kOutRgb>(form == kDwtSweep16, d_params, d_map, n, st);
-    else if (out_mode == kOutPlanes) go_inv_multi<1, kOutPlanes>(form == kDwtSweep16, d_params, d_map, n, st);
+    const bool h16 = form == kDwtSweep16;
+    if (out_mode == kOutRgb && channels == 3 && narrow) go_inv_multi<3, kOutRgb, true>(h16, d_params, d_map, n, st);
+    else if (out_mode == kOutRgb && channels == 3) go_inv_multi<3, kOutRgb, false>(h16, d_params, d_map, n, st);
+    else if (out_mode == kOutPlanes && narrow) go_inv_multi<1, kOutPlanes, true>(h16, d_params, d_map, n, st);
+    else if (out_mode == kOutPlanes) go_inv_multi<1, kOutPlanes, false>(h16, d_params, d_map, n, st);
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
@@ -817,7 +827,7 @@ cudaError_t launch_dwt_fwd(int mode, int channels, const FwdLevelParams& p0, cud
     if (channels != 1 && channels != 3) return cudaErrorInvalidValue;
     FwdLevelParams p = p0;
     unsigned gx, gy;
-    const int units = (int)dwt_fwd_grid(p, channels, kDwtSweep, gx, gy);
+    const int units = (int)sweep_grid(p.unit, p.sw, p.sh, channels, 0, false, gx, gy);
     if (mode == kSrcPlanes) go_fwd<kSrcPlanes>(p, units, st);
     else if (mode == kSrcRgbU8) go_fwd<kSrcRgbU8>(p, units, st);
     else if (mode == kSrcRgbF32) go_fwd<kSrcRgbF32>(p, units, st);
@@ -834,7 +844,7 @@ static void go_inv(const InvLevelParams& p, int units, cudaStream_t st) {
 cudaError_t launch_dwt_inv(int channels, int out_mode, const InvLevelParams& p0, cudaStream_t st) {
     InvLevelParams p = p0;
     unsigned gx, gy;
-    const int units = (int)dwt_inv_grid(p, out_mode == kOutPlanes ? channels : 1, kDwtSweep, gx, gy);
+    const int units = (int)sweep_grid(p.unit, p.sw, p.sh, out_mode == kOutPlanes ? channels : 1, 1, false, gx, gy);
     if (out_mode == kOutPlanes && (channels == 1 || channels == 3)) go_inv<1, kOutPlanes>(p, units, st);
     else if (out_mode == kOutRgb && channels == 3) go_inv<3, kOutRgb>(p, units, st);
     else return cudaErrorInvalidValue;
@@ -970,8 +980,8 @@ cudaError_t dwt_autotune(int dev, float fwd_ms[9], float inv_ms[9], int* fwd_bes
             if (e != cudaSuccess) return done(e);
             for (int rep = 0; rep < 6; rep++) {
                 if (rep == 1 && (e = cudaEventRecord(e0, st)) != cudaSuccess) return done(e);
-                e = inv ? launch_dwt_inv_multi(1, kOutPlanes, (const InvLevelParams*)dpi, map, units, kDwtSweep, st)
-                        : launch_dwt_fwd_multi(kSrcRgbU8, 1, (const FwdLevelParams*)dp, map, units, kDwtSweep, st);
+                e = inv ? launch_dwt_inv_multi(1, kOutPlanes, (const InvLevelParams*)dpi, map, units, kDwtSweep, false, st)
+                        : launch_dwt_fwd_multi(kSrcRgbU8, 1, (const FwdLevelParams*)dp, map, units, kDwtSweep, false, st);
                 if (e != cudaSuccess) return done(e);
             }
             if ((e = cudaEventRecord(e1, st)) != cudaSuccess) return done(e);

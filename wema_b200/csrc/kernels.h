@@ -170,10 +170,11 @@ cudaError_t launch_window(const WindowParams& wp, int channels, cudaStream_t st)
 enum { kDwtSweep = 0, kDwtSweep16 = 1, kDwtTiles = 2, kDwtTiles16 = 3 };
 unsigned dwt_fwd_grid(FwdLevelParams& p, int channels_z, int form, unsigned& gx, unsigned& gy);
 unsigned dwt_inv_grid(InvLevelParams& p, int channels_z, int form, unsigned& gx, unsigned& gy);
+bool dwt_narrow(int sw);        // a level of sw pairs is at most two strips wide: some task is, the launch is `narrow`
 cudaError_t launch_dwt_fwd_multi(int mode, int channels, const FwdLevelParams* d_params, const int* d_map, unsigned blocks,
-                                 int form, cudaStream_t st);
+                                 int form, bool narrow, cudaStream_t st);
 cudaError_t launch_dwt_inv_multi(int channels, int out_mode, const InvLevelParams* d_params,
-                                 const int* d_map, unsigned blocks, int form, cudaStream_t st);
+                                 const int* d_map, unsigned blocks, int form, bool narrow, cudaStream_t st);
 // the tiles (dwt_tiles.cu), behind the functions above
 cudaError_t tiles_prepare_device();
 unsigned tiles_grid(int sw, int sh, int channels_z, unsigned& gx, unsigned& gy);

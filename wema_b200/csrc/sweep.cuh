@@ -39,14 +39,22 @@ inline __host__ __device__ int sweep_groups(int pairs, int q) {
     const int most = sweep_across(pairs, q) * SW_LANES * q;
     return (pairs + most - 1) / most;
 }
-// this warp's part of rows ya .. yb - 1 that its CTA takes
+// this warp's strip and rows of rows a .. b - 1 of a CTA's group of strips
+template <bool NARROW>
 struct WarpRows {
-    int strip, ya, yb;                   // (of the CTA's strips, of the rows)
-    __device__ __forceinline__ WarpRows(int across, int a, int b) {
-        const int w = threadIdx.x >> 5, down = SW_WARPS / across, r = w / across;
-        strip = w % across;
-        ya = a + (b - a) * r / down;
-        yb = a + (b - a) * (r + 1) / down;
+    int strip, ya, yb;
+    __device__ __forceinline__ WarpRows(int group, int across, int a, int b) {
+        const int w = threadIdx.x >> 5;
+        if constexpr (NARROW) {
+            const int down = SW_WARPS / across, r = w / across;
+            strip = group * across + w % across;
+            ya = a + (b - a) * r / down;
+            yb = a + (b - a) * (r + 1) / down;
+        } else {
+            strip = group * SW_WARPS + w;
+            ya = a;
+            yb = b;
+        }
     }
 };
 
