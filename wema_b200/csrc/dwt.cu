@@ -817,6 +817,33 @@ cudaError_t launch_dwt_inv_multi(int channels, int out_mode, const InvLevelParam
     return cudaGetLastError();
 }
 
+// ---- one stream's level: by tiles (dwt_tiles.cu) or by sweeps.  A sweep's chain of
+// steps (rows of a segment + 4) is longer than a tile's, so a level that does not
+// fill the GPU several times over is a tile's; with other frames in flight the
+// sweeps' fewer instructions count, which draws the lines for one channel
+// lower.  Level alone, tiles / sweeps, us: forward from RGB24 1280x720 8.3 / 12.8,
+// colour 17.0 / 21.8; 1920x1080 12.4 / 16.3, colour 27.1 / 33.4; 3840x2160 35.8 /
+// 34.9, colour 77 / 92; 320x240 colour 13.6 / 10.8; planes of 640x360 5.0 / 7.0,
+// 1920x1080 9.3 / 10.4, three of them 22.4 / 18.5.  Inverse 1280x720 6.2 / 6.6,
+// 1920x1080 10.0 / 7.6, three planes of 960x540 7.8 / 8.7, of 1280x720 12.6 / 11.3;
+// to RGB 1280x720 16.1 / 11.9, 1366x767 (rows that do not start at words) 14.5 /
+// 16.9, 427x239 11.6 / 8.9.  Frames in flight, before -> with the lines: 1366x767
+// colour 88 -> 68, 1920x1080 colour 111 -> 107, with FP16 planes 1281x719 colour
+// 81 -> 61, 640x480 colour 50 -> 42, 1280x720 64 -> 60; past the lines 1920x1080
+// luma would go 83 -> 86, 3840x2160 colour 364 -> 368.  A level at most two strips
+// wide leaves half of a CTA's warps idle: 33x30000 244 -> 79 in colour.
+static bool fwd_by_tiles(int mode, int channels, const FwdLevelParams& p) {
+    const long long px = (long long)p.iw * p.ih;
+    if (channels == 3 && mode != kSrcPlanes) return px >= 200000 && (px < 4000000 || dwt_narrow(p.sw));
+    return px < (channels == 1 ? 600000 : 1000000) || dwt_narrow(p.sw);
+}
+static bool inv_by_tiles(int channels, int out_mode, const InvLevelParams& p) {
+    const long long px = (long long)p.ow * p.oh;
+    if (out_mode == kOutRgb)
+        return px >= 250000 && (dwt_narrow(p.sw) || ((p.ow & 3) && (p.out_f32 || px < 4000000)));
+    return px < (channels == 1 ? 1200000 : 640000) || dwt_narrow(p.sw);
+}
+
 template <int MODE>
 static void go_fwd(const FwdLevelParams& p, int units, cudaStream_t st) {
     const int n = ctas_for(units, 0, fwd_res(MODE, false));
@@ -825,6 +852,7 @@ static void go_fwd(const FwdLevelParams& p, int units, cudaStream_t st) {
 }
 cudaError_t launch_dwt_fwd(int mode, int channels, const FwdLevelParams& p0, cudaStream_t st) {
     if (channels != 1 && channels != 3) return cudaErrorInvalidValue;
+    if (fwd_by_tiles(mode, channels, p0)) return launch_tiles_fwd(mode, channels, p0, st);
     FwdLevelParams p = p0;
     unsigned gx, gy;
     const int units = (int)sweep_grid(p.unit, p.sw, p.sh, channels, 0, false, gx, gy);
@@ -842,6 +870,7 @@ static void go_inv(const InvLevelParams& p, int units, cudaStream_t st) {
     else k_dwt_inv<C, OUT, false><<<n, SW_THREADS, 0, st>>>(p, units);
 }
 cudaError_t launch_dwt_inv(int channels, int out_mode, const InvLevelParams& p0, cudaStream_t st) {
+    if (inv_by_tiles(channels, out_mode, p0)) return launch_tiles_inv(channels, out_mode, p0, st);
     InvLevelParams p = p0;
     unsigned gx, gy;
     const int units = (int)sweep_grid(p.unit, p.sw, p.sh, out_mode == kOutPlanes ? channels : 1, 1, false, gx, gy);
@@ -852,17 +881,19 @@ cudaError_t launch_dwt_inv(int channels, int out_mode, const InvLevelParams& p0,
 }
 
 // Whether levels from one of sw x sh positions on run in a cluster: at most 6 rows
-// of a strip per warp.  A stream's frame, levels apart -> in a cluster: 320x240
-// (1.2 rows) 49 -> 43 us, colour 42 -> 36; 853x479 (5.0) 64 -> 59, colour
-// 65 -> 56; 1023x577 (7.6) 63 -> 65, colour 66 -> 72; 1920x1080 (22.5) 82 -> 98:
-// from about 7 rows on the whole GPU is faster than a cluster's 8 SMs.
-constexpr int TAIL_ROWS = 6;
-static bool tail_fits(int sw, int sh, int n) {
+// of a strip per warp, in colour 2.  The cluster saves two launches of the host per
+// direction, and is the longer chain on the GPU (levels of 640x480 luma 21 us, by
+// tiles 14).  So it is the faster one where the host bounds the frames in flight:
+// luma 320x240 (1.2 rows) 47 -> 42 us a frame, 640x480 49.8 -> 49.5, with FP16
+// planes 60 -> 49; in colour, whose forward levels bound the frame, 160x120 35 -> 32,
+// 320x240 40 -> 39, but 640x360 (2.8 rows) 42 -> 45, 640x480 44 -> 47.
+constexpr int TAIL_ROWS = 6, TAIL_ROWS_COLOR = 2;
+static bool tail_fits(int sw, int sh, int n, int channels) {
     const long long rows = (long long)((sw + SW_LANES * SQ - 1) / (SW_LANES * SQ)) * sh;
-    return n >= 2 && n <= 3 && rows <= TAIL_ROWS * TAIL_CTAS * TAIL_WARPS;
+    return n >= 2 && n <= 3 && rows <= (channels == 3 ? TAIL_ROWS_COLOR : TAIL_ROWS) * TAIL_CTAS * TAIL_WARPS;
 }
 cudaError_t launch_dwt_fwd_levels(int channels, const FwdLevelParams* p, int n, cudaStream_t st, int* launches) {
-    if (n > 0 && tail_fits(p[0].sw, p[0].sh, n)) {
+    if (n > 0 && tail_fits(p[0].sw, p[0].sh, n, channels)) {
         LevelTail<FwdLevelParams> t{};
         for (int l = 0; l < n; l++) t.lv[l] = p[l];
         t.count = n;
@@ -878,7 +909,7 @@ cudaError_t launch_dwt_fwd_levels(int channels, const FwdLevelParams* p, int n, 
     return e;
 }
 cudaError_t launch_dwt_inv_levels(int channels, const InvLevelParams* p, int n, cudaStream_t st, int* launches) {
-    if (n > 0 && tail_fits(p[n - 1].sw, p[n - 1].sh, n)) {
+    if (n > 0 && tail_fits(p[n - 1].sw, p[n - 1].sh, n, channels)) {
         LevelTail<InvLevelParams> t{};
         for (int l = 0; l < n; l++) t.lv[l] = p[l];
         t.count = n;

@@ -1,6 +1,6 @@
 // dwt_tiles.cu - the DWT levels by tiles: where the sweeps of dwt.cu are the slower
 // form: batched launches that hold FP64 filter state or differ in storage type
-// (batch.h has the rule).
+// (batch.h has the rule), and small levels of one stream (dwt.cu has it).
 //
 // A CTA owns a tile of TP x TP subband pairs (TP = 27) and stages a 64 x 64
 // sample region - the tile's 54 samples plus a 4-sample halo before and a
@@ -578,6 +578,20 @@ __device__ __forceinline__ void dwt_inv_body(const InvLevelParams& p, int bx, in
 }
 
 // ------------------------------------------------------------- wrappers
+// One stream per launch: compiled for its plane type.  4 CTAs per SM of one channel
+// (colour 3) asked of the register allocator; forward 3.
+template <int C, int MODE, bool H16>
+__global__ void __launch_bounds__(DWT_THREADS, 3) k_tiles_fwd(FwdLevelParams p) {
+    if (!H16 && fwd_full(p, blockIdx.x, blockIdx.y))
+        dwt_fwd_body<C, MODE, false, true>(p, blockIdx.x, blockIdx.y, blockIdx.z);
+    else dwt_fwd_body<C, MODE, H16, false>(p, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+template <int C, int OUT, bool H16>
+__global__ void __launch_bounds__(DWT_THREADS, C == 1 ? 4 : 3) k_tiles_inv(InvLevelParams p) {
+    if (!H16 && inv_full(p, blockIdx.x, blockIdx.y))
+        dwt_inv_body<C, OUT, false, true>(p, blockIdx.x, blockIdx.y, blockIdx.z);
+    else dwt_inv_body<C, OUT, H16, false>(p, blockIdx.x, blockIdx.y, blockIdx.z);
+}
 // Batched (task = stream, the map counts tiles).  ANY16: some task has FP16 planes,
 // chosen per CTA; a kernel holding both bodies is allocated registers for both.
 // A one-channel CTA works on channel z of its task: the task's parameters copied
@@ -642,10 +656,43 @@ unsigned tiles_grid(int sw, int sh, int channels_z, unsigned& gx, unsigned& gy) 
 cudaError_t tiles_prepare_device() {
     cudaError_t e = cudaSuccess;
     for (const void* k :
-         {(const void*)k_tiles_fwd_multi<3, kSrcRgbU8, false>, (const void*)k_tiles_fwd_multi<3, kSrcRgbU8, true>,
+         {(const void*)k_tiles_fwd<3, kSrcRgbU8, false>, (const void*)k_tiles_fwd<3, kSrcRgbU8, true>,
+          (const void*)k_tiles_fwd<3, kSrcRgbF32, false>, (const void*)k_tiles_fwd<3, kSrcRgbF32, true>,
+          (const void*)k_tiles_inv<3, kOutRgb, false>, (const void*)k_tiles_inv<3, kOutRgb, true>,
+          (const void*)k_tiles_fwd_multi<3, kSrcRgbU8, false>, (const void*)k_tiles_fwd_multi<3, kSrcRgbU8, true>,
           (const void*)k_tiles_inv_multi<3, kOutRgb>})
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tiles_smem(3));
     return e;
+}
+
+template <int C, int MODE>
+static void go_fwd(const FwdLevelParams& p, int z, cudaStream_t st) {
+    const dim3 grid(tiles_of(p.sw), tiles_of(p.sh), (unsigned)z);
+    if (p.h16) k_tiles_fwd<C, MODE, true><<<grid, DWT_THREADS, tiles_smem(C), st>>>(p);
+    else k_tiles_fwd<C, MODE, false><<<grid, DWT_THREADS, tiles_smem(C), st>>>(p);
+}
+cudaError_t launch_tiles_fwd(int mode, int channels, const FwdLevelParams& p, cudaStream_t st) {
+    if (channels != 1 && channels != 3) return cudaErrorInvalidValue;
+    if (mode == kSrcPlanes) go_fwd<1, kSrcPlanes>(p, channels, st);
+    else if (mode == kSrcRgbU8 && channels == 3) go_fwd<3, kSrcRgbU8>(p, 1, st);
+    else if (mode == kSrcRgbU8) go_fwd<1, kSrcRgbU8>(p, 1, st);
+    else if (mode == kSrcRgbF32 && channels == 3) go_fwd<3, kSrcRgbF32>(p, 1, st);
+    else if (mode == kSrcRgbF32) go_fwd<1, kSrcRgbF32>(p, 1, st);
+    else return cudaErrorInvalidValue;
+    return cudaGetLastError();
+}
+
+template <int C, int OUT>
+static void go_inv(const InvLevelParams& p, int z, cudaStream_t st) {
+    const dim3 grid(tiles_of(p.sw), tiles_of(p.sh), (unsigned)z);
+    if (p.h16) k_tiles_inv<C, OUT, true><<<grid, DWT_THREADS, tiles_smem(C), st>>>(p);
+    else k_tiles_inv<C, OUT, false><<<grid, DWT_THREADS, tiles_smem(C), st>>>(p);
+}
+cudaError_t launch_tiles_inv(int channels, int out_mode, const InvLevelParams& p, cudaStream_t st) {
+    if (out_mode == kOutPlanes && (channels == 1 || channels == 3)) go_inv<1, kOutPlanes>(p, channels, st);
+    else if (out_mode == kOutRgb && channels == 3) go_inv<3, kOutRgb>(p, 1, st);
+    else return cudaErrorInvalidValue;
+    return cudaGetLastError();
 }
 
 template <int C, int MODE>

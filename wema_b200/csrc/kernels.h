@@ -175,9 +175,11 @@ cudaError_t launch_dwt_fwd_multi(int mode, int channels, const FwdLevelParams* d
                                  int form, bool narrow, cudaStream_t st);
 cudaError_t launch_dwt_inv_multi(int channels, int out_mode, const InvLevelParams* d_params,
                                  const int* d_map, unsigned blocks, int form, bool narrow, cudaStream_t st);
-// the tiles (dwt_tiles.cu), behind the functions above
+// the tiles (dwt_tiles.cu), behind the functions above and launch_dwt_fwd / _inv
 cudaError_t tiles_prepare_device();
 unsigned tiles_grid(int sw, int sh, int channels_z, unsigned& gx, unsigned& gy);
+cudaError_t launch_tiles_fwd(int mode, int channels, const FwdLevelParams& p, cudaStream_t st);
+cudaError_t launch_tiles_inv(int channels, int out_mode, const InvLevelParams& p, cudaStream_t st);
 cudaError_t launch_tiles_fwd_multi(int mode, int channels, const FwdLevelParams* d_params, const int* d_map,
                                    unsigned blocks, bool any16, cudaStream_t st);
 cudaError_t launch_tiles_inv_multi(int channels, int out_mode, const InvLevelParams* d_params, const int* d_map,
