@@ -902,11 +902,11 @@ cudaError_t launch_passthrough(const TransferParams& p, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// ---- the autotuner's trial of the segment height: one launch of the sweep
-// over a 3840 x 8640 RGB24 frame (four 2160-row frames' worth of strips and
-// segments, about the batched tick's warp count at 128 rows), each candidate
-// timed over five launches after one warm-up (the default, 64, as the even
-// split it stands for); the fastest is kept.  Outputs do not depend on the
+// ---- the autotuner's trial of the batched sweep's segment height: a 3840 x 8640
+// RGB24 frame (four 2160-row frames' worth of strips and segments, about the
+// batched tick's warp count at 128 rows) as one task of the batched launch, each
+// candidate set on the device as a tick would find it and timed over five
+// launches after one warm-up; the fastest is kept.  Outputs do not depend on the
 // choice.
 cudaError_t guided_autotune(int dev, const int* cand, int nc, float* ms, int* chosen) {
     cudaError_t e = cudaSetDevice(dev);
@@ -915,40 +915,50 @@ cudaError_t guided_autotune(int dev, const int* cand, int nc, float* ms, int* ch
     const size_t P = (size_t)W * H;
     uint8_t *in = nullptr, *out = nullptr;
     float* gray = nullptr;
+    void *dp = nullptr, *dmap = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaStream_t st = nullptr;
+    const int keep = guided_rows(dev);
     auto done = [&](cudaError_t r) {
-        if (in) cudaFree(in);
-        if (out) cudaFree(out);
-        if (gray) cudaFree(gray);
+        for (void* p : {(void*)in, (void*)out, (void*)gray, dp, dmap})
+            if (p) cudaFree(p);
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
         if (st) cudaStreamDestroy(st);
+        if (r != cudaSuccess) guided_set_rows(dev, keep);   // leave the device's choice as it was
         return r;
     };
     if ((e = cudaMalloc(&in, 3 * P)) != cudaSuccess) return done(e);
     if ((e = cudaMalloc(&out, 3 * P)) != cudaSuccess) return done(e);
     if ((e = cudaMalloc(&gray, P * sizeof(float))) != cudaSuccess) return done(e);
+    if ((e = cudaMalloc(&dp, sizeof(TransferParams))) != cudaSuccess) return done(e);
+    if ((e = cudaMalloc(&dmap, 8 * sizeof(int))) != cudaSuccess) return done(e);
     if ((e = cudaMemset(in, 0x5a, 3 * P)) != cudaSuccess) return done(e);
     if ((e = cudaMemset(gray, 0, P * sizeof(float))) != cudaSuccess) return done(e);
     if ((e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)) != cudaSuccess) return done(e);
     if ((e = cudaEventCreate(&e0)) != cudaSuccess || (e = cudaEventCreate(&e1)) != cudaSuccess) return done(e);
     if ((e = spatial_prepare_device()) != cudaSuccess) return done(e);
-    int best = guided_rows(dev);
+    int best = keep;
     float best_ms = 1e30f;
     for (int k = 0; k < nc; k++) {
-        SpArgs a{};
-        a.p.w = W;
-        a.p.h = H;
-        a.p.vec_end = (long long)P;
-        a.p.src_u8 = in;
-        a.p.gray_out = gray;
-        a.p.out_u8 = out;
-        a.p.edge_aware = 1;
-        a.p.seg_rows = cand[k] == GS_ROWS_DEFAULT ? 0 : cand[k];
+        guided_set_rows(dev, cand[k]);
+        TransferParams tp{};
+        tp.w = W;
+        tp.h = H;
+        tp.vec_end = (long long)P;
+        tp.src_u8 = in;
+        tp.gray_out = gray;
+        tp.out_u8 = out;
+        tp.edge_aware = 1;
+        unsigned gx, gy;
+        const unsigned units = transfer_grid(tp, gx, gy);
+        const int map[5] = {1, 0, (int)units, (int)gx, (int)gy};
+        if ((e = cudaMemcpy(dp, &tp, sizeof tp, cudaMemcpyHostToDevice)) != cudaSuccess) return done(e);
+        if ((e = cudaMemcpy(dmap, map, sizeof map, cudaMemcpyHostToDevice)) != cudaSuccess) return done(e);
         for (int rep = 0; rep < 6; rep++) {
             if (rep == 1 && (e = cudaEventRecord(e0, st)) != cudaSuccess) return done(e);
-            if ((e = launch_transfer(a.p, st)) != cudaSuccess) return done(e);
+            e = launch_transfer_multi(1, (const TransferParams*)dp, (const int*)dmap, units, transfer_rows_mode(tp), st);
+            if (e != cudaSuccess) return done(e);
         }
         if ((e = cudaEventRecord(e1, st)) != cudaSuccess) return done(e);
         if ((e = cudaEventSynchronize(e1)) != cudaSuccess) return done(e);
