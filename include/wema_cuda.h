@@ -307,18 +307,19 @@ int wema_cuda_server_stats(wema_cuda_server *srv, int reset, wema_cuda_serve_sta
  *     warps (the setting 64, the default) and at 128 and 256 output rows per
  *     segment (a 3840x8640 trial frame) and keeps the fastest;
  *   - the batched luma DWT level-0 kernels, forward and inverse, in nine
- *     variants each: at most {3, 4, 5} CTAs per SM (fewer where fewer fit) x
- *     units of {1, 2, 4} pairs of rows (variant = 3 * index + index; a
+ *     variants each: at most {2, 3, 4} CTAs per SM forward, {3, 4, 5} inverse
+ *     x units of {1, 2, 4} pairs of rows (variant = 3 * index + index; a
  *     3840x4320 trial frame, the forward with the temporal filter's step
  *     inside as steady batched ticks run it) and keeps the fastest of each
- *     (5 x 2 for both until then);
+ *     (4 x 2 and 5 x 2 until then);
  * allocating ~950 MB for the trials (one at a time) and freeing it.  Every
- * later launch on the device uses the choices.  Returns the positions per
+ * later launch of these kernels on the device uses the choices (one stream's
+ * guided sweep splits its rows by itself).  Returns the positions per
  * thread (or -1) and writes the timings to `report` (may be NULL; 1 KiB is
  * enough).  Results do not depend on any choice - each position's and each
  * pixel's arithmetic is the same - only speed does.  set / get fix or read a
- * choice directly (positions 2, 4 or 8; rows a multiple of 16 in 16..4096;
- * DWT variant 0..8, inverse = 0 forward, 1 inverse). */
+ * choice directly (positions 2, 4 or 8; rows a multiple of 16 in 16..4096,
+ * of which 64 stands for the even split; DWT variant 0..8, inverse = 0 forward, 1 inverse). */
 int wema_cuda_autotune(int device, char *report, size_t cap);
 int wema_cuda_set_iir_positions(int device, int positions);
 int wema_cuda_get_iir_positions(int device);

@@ -1,5 +1,6 @@
 """The autotuner times the launches that its choices steer: each candidate's trial
-of the guided sweep is the launch that a tick with that setting issues."""
+of the guided sweep is the launch that a tick with that setting issues, and the
+nine variants of the forward and of the inverse level-0 transform differ in it."""
 import json
 
 import pytest
@@ -53,3 +54,14 @@ def test_guided_trials(settings, tmp_path):
     b.close()
     assert len(ticked) == 3
     assert trials == [x for x in ticked for _ in range(6)]
+
+
+def test_dwt_variants_differ(settings, tmp_path):
+    wc.autotune(0)
+    got = launches_of(lambda: wc.autotune(0), tmp_path)
+    for kernel in ("k_dwt_fwd_multi", "k_dwt_inv_multi"):
+        trials = [g for n, g in got if kernel in n]
+        assert len(trials) == 54                 # nine variants, a warm-up and five launches each
+        grids = [trials[6 * v] for v in range(9)]
+        for unit in range(3):                    # three limits of CTAs per SM at each unit
+            assert len({grids[3 * i + unit] for i in range(3)}) == 3, f"{kernel}: {grids}"

@@ -687,9 +687,10 @@ __global__ void __launch_bounds__(SW_THREADS, inv_res(C))
 }
 
 // ---- tuning of the batched sweeps, per device: variant v = 3 * i + k, at most
-// kRes[i] CTAs per SM (fewer where fewer fit) in units of kUnit[k] pairs of rows
+// kRes[inverse][i] CTAs per SM in units of kUnit[k] pairs of rows; the most is what
+// fits of the one-channel kernels (the colour inverse fits 2 whatever is set)
 constexpr int kDwtVariants = 9;
-static const int kRes[3] = {3, 4, 5}, kUnit[3] = {1, 2, 4};
+static const int kRes[2][3] = {{2, 3, 4}, {3, 4, 5}}, kUnit[3] = {1, 2, 4};
 static std::atomic<int> g_dwt_var[64][2];     // [device][0 forward, 1 inverse], value + 1
 
 static int dwt_dev_now() {
@@ -699,15 +700,15 @@ static int dwt_dev_now() {
 }
 int dwt_variant(int dev, int inverse) {
     const int v = (dev >= 0 && dev < 64) ? g_dwt_var[dev][inverse ? 1 : 0].load() : 0;
-    return v > 0 ? v - 1 : 2 * 3 + 1;         // until tuned: 5 CTAs per SM, 2 pairs of rows
+    return v > 0 ? v - 1 : 2 * 3 + 1;         // until tuned: the most CTAs per SM, 2 pairs of rows
 }
 bool dwt_set_variant(int dev, int inverse, int v) {
     if (dev < 0 || dev >= 64 || v < 0 || v >= kDwtVariants) return false;
     g_dwt_var[dev][inverse ? 1 : 0].store(v + 1);
     return true;
 }
-void dwt_variant_shape(int v, int* res, int* unit) {
-    *res = kRes[v / 3];
+void dwt_variant_shape(int v, int inverse, int* res, int* unit) {
+    *res = kRes[inverse ? 1 : 0][v / 3];
     *unit = kUnit[v % 3];
 }
 
@@ -731,16 +732,18 @@ static int sweep_ctas(int units, int unit, int res) {
     }
     return best;
 }
-static int ctas_for(int units, int inverse, int most) {
+// more: CTAs per SM above the setting's (one stream's forward, without the filter's
+// rings, fits one more than the batched)
+static int ctas_for(int units, int inverse, int most, int more = 0) {
     int res, unit;
-    dwt_variant_shape(dwt_variant(dwt_dev_now(), inverse), &res, &unit);
-    return sweep_ctas(units, unit, std::min(res, most));
+    dwt_variant_shape(dwt_variant(dwt_dev_now(), inverse), inverse, &res, &unit);
+    return sweep_ctas(units, unit, std::min(res + more, most));
 }
 
 // ----------------------------------------------------------------- launch
 static unsigned sweep_grid(int& unit, int sw, int sh, int channels_z, int inverse, bool narrow, unsigned& gx, unsigned& gy) {
     int res;
-    dwt_variant_shape(dwt_variant(dwt_dev_now(), inverse), &res, &unit);
+    dwt_variant_shape(dwt_variant(dwt_dev_now(), inverse), inverse, &res, &unit);
     if (narrow) unit *= SW_WARPS / sweep_across(sw, SQ);   // (a warp's rows stay the setting's)
     gx = (unsigned)((sh + unit - 1) / unit);
     gy = (unsigned)sweep_groups(sw, SQ);
@@ -846,7 +849,7 @@ static bool inv_by_tiles(int channels, int out_mode, const InvLevelParams& p) {
 
 template <int MODE>
 static void go_fwd(const FwdLevelParams& p, int units, cudaStream_t st) {
-    const int n = ctas_for(units, 0, fwd_res(MODE, false));
+    const int n = ctas_for(units, 0, fwd_res(MODE, false), 1);
     if (p.h16) k_dwt_fwd<MODE, true><<<n, SW_THREADS, 0, st>>>(p, units);
     else k_dwt_fwd<MODE, false><<<n, SW_THREADS, 0, st>>>(p, units);
 }

@@ -59,11 +59,11 @@ cudaError_t launch_dwt_inv(int channels, int out_mode, const InvLevelParams& p, 
 // first), planes in and out; *launches: how many it took
 cudaError_t launch_dwt_fwd_levels(int channels, const FwdLevelParams* p, int n, cudaStream_t st, int* launches);
 cudaError_t launch_dwt_inv_levels(int channels, const InvLevelParams* p, int n, cudaStream_t st, int* launches);
-// tuning variant (0..8) of the DWT sweeps on a device: at most {3, 4, 5}[v / 3]
-// CTAs per SM, units of {1, 2, 4}[v % 3] pairs of rows
+// tuning variant (0..8) of the DWT sweeps on a device: at most {2, 3, 4}[v / 3]
+// CTAs per SM forward, {3, 4, 5}[v / 3] inverse, units of {1, 2, 4}[v % 3] pairs of rows
 int dwt_variant(int dev, int inverse);
 bool dwt_set_variant(int dev, int inverse, int v);
-void dwt_variant_shape(int v, int* res, int* unit);
+void dwt_variant_shape(int v, int inverse, int* res, int* unit);
 // times every variant of the forward and inverse level-0 luma kernels, keeps the fastest
 cudaError_t dwt_autotune(int dev, float fwd_ms[9], float inv_ms[9], int* fwd_best, int* inv_best);
 

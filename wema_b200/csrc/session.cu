@@ -758,12 +758,12 @@ WEMA_API int wema_cuda_autotune(int device, char* report, size_t cap) {
                           inv ? "inverse" : "forward");
             for (int v = 0; v < 9 && n > 0 && (size_t)n < cap; v++) {
                 int mb, lp;
-                dwt_variant_shape(v, &mb, &lp);
+                dwt_variant_shape(v, inv, &mb, &lp);
                 n += snprintf(report + n, cap - n, " %dx%d %.4f", mb, lp, t[v]);
             }
             if (n > 0 && (size_t)n < cap) {
                 int mb, lp;
-                dwt_variant_shape(inv ? ibest : fbest, &mb, &lp);
+                dwt_variant_shape(inv ? ibest : fbest, inv, &mb, &lp);
                 n += snprintf(report + n, cap - n, " ms -> %dx%d", mb, lp);
             }
         }
