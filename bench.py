@@ -78,10 +78,10 @@ METRIC = "Mpix-frames/s"
 # the 48-stream tick; the threshold of the plain workload is monoids + walk.
 _MIX = 77.722 / 19.046
 TRAFFIC_NCU = {
-    ("mixed_streams_48", "fwd_dwt_level0"): int((288116224 + 304738048) * _MIX),
-    ("mixed_streams_48", "luma_transfer"): int((148669184 + 34321152) * _MIX),
-    ("mixed_streams_48", "inv_dwt_level0"): int((133352960 + 47001344) * _MIX),
-    ("plain_fullhd_color", "threshold"): 25081088 + 2323456,
+    ("mixed_streams_48", "fwd_dwt_level0"): int((293729280 + 305726208) * _MIX),
+    ("mixed_streams_48", "luma_transfer"): int((182076416 + 38378752) * _MIX),
+    ("mixed_streams_48", "inv_dwt_level0"): int((150262528 + 46534144) * _MIX),
+    ("plain_fullhd_color", "threshold"): 25011712 + 2315008,
 }
 
 
@@ -210,23 +210,24 @@ def stage_bytes(w, h, channels, levels_dims, pu, fused=True):
 
 # kernels behind each stage of a batched tick (one launch per tick over every stream)
 STAGE_KERNELS_MULTI = {
-    "fwd_dwt_level0": "k_dwt_fwd_multi<1,1> (level 0, RGB in, with the IIR step)",
-    "fwd_dwt_levels": "k_dwt_fwd_multi<1,0> x 3 (with the IIR step)",
+    "fwd_dwt_level0": "k_dwt_fwd_multi (level 0, RGB in, with the IIR step)",
+    "fwd_dwt_levels": "k_dwt_fwd_multi x 3 (with the IIR step)",
     "threshold": "k_thr_monoids_multi + k_thr_walk_multi",
     "temporal_amplify": "k_iir_multi (first frames only; else inside the forward transform)",
-    "inv_dwt_levels": "k_dwt_inv_multi<1,0> x 3",
-    "inv_dwt_level0": "k_dwt_inv_multi<1,0> (level 0)",
+    "inv_dwt_levels": "k_dwt_inv_multi x 3",
+    "inv_dwt_level0": "k_dwt_inv_multi (level 0)",
     "luma_transfer": "k_guided_transfer_multi",
 }
 
-# kernels behind each stage (one launch per frame unless noted)
+# kernels behind each stage (one launch per frame unless noted; the transforms
+# by tiles or by sweeps, whichever is the faster at the level's size)
 STAGE_KERNELS = {
-    "fwd_dwt_level0": "k_dwt_fwd<1|2> (level 0, RGB in)",
-    "fwd_dwt_levels": "k_dwt_fwd<0> x (levels - 1)",
+    "fwd_dwt_level0": "k_tiles_fwd / k_dwt_fwd (level 0, RGB in)",
+    "fwd_dwt_levels": "k_tiles_fwd / k_dwt_fwd x (levels - 1), or k_dwt_fwd_tail",
     "threshold": "k_thr_monoids + k_thr_walk",
     "temporal_amplify": "k_iir x channels",
-    "inv_dwt_levels": "k_dwt_inv<1,0> x (levels - 1)",
-    "inv_dwt_level0": "k_dwt_inv<3,1> (colour, RGB out) / k_dwt_inv<1,0> (luma)",
+    "inv_dwt_levels": "k_tiles_inv / k_dwt_inv x (levels - 1), or k_dwt_inv_tail",
+    "inv_dwt_level0": "k_dwt_inv / k_tiles_inv (planes out; colour: RGB out)",
     "luma_transfer": "k_guided_transfer / k_gauss_transfer",
 }
 

@@ -14,13 +14,14 @@
 // separate multiplies (dwt.c:45-170 as GCC -Ofast evaluates it), so
 // coefficients are bit-exact.
 //
-// What bounds them: HBM and issue slots at the large levels, the chain of steps of
-// a short segment at the small ones.  Measured against kernels that staged
-// 64x64 regions in shared memory and wrote 54x54 of them (1.4 times the area,
-// 80 instructions per pixel of the inverse against 32 here):
-//   3840x4320, level 0   forward 55 -> 37 us (bytes in, planes out), with the
-//                        filter's step 140 -> 118; inverse 55 -> 41
-//   the 48-stream tick   inverse level 0 279 -> 173 us, levels 3..1 116 -> 81
+// What bounds them: the latency of their loads and HBM at the large levels, the
+// chain of steps of a short segment at the small ones, which are a tile's
+// (dwt_tiles.cu) where that is the faster form.  Measured against the tiles, which
+// load and lift 1.4 times the area through shared memory (thread instructions per
+// pixel: forward with the filter's step 93 against 171, inverse 37 against 91):
+//   3840x4320, level 0   forward with the filter's step 140 -> 118 us; inverse 55 -> 42
+//   the 48-stream tick   level 0 forward 0.615 -> 0.578 ms, inverse 0.279 -> 0.182,
+//                        levels 3..1 inverse 0.116 -> 0.088
 #include <algorithm>
 #include <atomic>
 #include <type_traits>

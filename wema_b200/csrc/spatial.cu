@@ -79,14 +79,13 @@ __device__ __forceinline__ void store_rgb(const TransferParams& p, int pi, float
 // where its segment starts: any segment that starts at a multiple of 16 rows
 // gives bit-identical output, and rounding drift spans at most 15 slides.
 //
-// What bounds it: instruction latency at 12 warps per SM (18.4 KB of rings per
-// warp) - 437 instructions per row of a strip at 61% of the issue slots, DRAM
-// at 12%.  So the work per pixel is cut (fewer halo rows by segments as long
+// What bounds it: instruction issue and latency at 12 warps per SM (18.4 KB of
+// rings per warp) - 460 instructions per row of a strip at 64% of the issue slots,
+// DRAM at 19%.  So the work per pixel is cut (fewer halo rows by segments as long
 // as an even split allows, quant12, shared quad sums) and the loop body is
 // kept in few branch-free pieces: rows come in pairs whose second never
 // recomputes its sums.  A 3840x8640 frame: 203 us against 248 (fixed segments
-// of 64 rows, every byte through the float steps); 221 of them with fixed
-// segments still.
+// of 64 rows, every byte through the float steps); fixed segments of 128 rows 241.
 constexpr int GR = 4;                   // guided-filter radius (wema.c:314)
 constexpr int GS_IN = 128;              // input columns per strip (4 per lane)
 constexpr int GS_OUT = GS_IN - 4 * GR;  // output columns per strip
@@ -199,7 +198,7 @@ __device__ __forceinline__ void guide4(const float (&c)[12], const float (&gy)[4
 // of the pixel are b + n clamped with n = round(255 dy): two channels per
 // 16-bit-pair add, minimum and maximum.  A warp with another pixel (about one
 // row in 40) takes the float steps for the lanes that hold one; the clamps
-// send a NaN to 0 (SAT) or 255.  45 instead of 93 instructions per 4 pixels.
+// send a NaN to 0 (SAT) or 255.
 template <bool SAT>
 __device__ __forceinline__ void quant12(const uint32_t (&w)[3], const float (&dy)[4], uint32_t (&o)[3]) {
     constexpr float M = 12582912.0f;    // 1.5 * 2^23: the low bits of x + M hold round(x)
