@@ -1,5 +1,5 @@
 """A stream's levels by tiles or by sweeps: frames on either side of each line
-between them (luma 0.6 and 1.2 million pixels; colour 0.2, 0.25, 0.64, 1 and 4
+between them (luma 0.6, 1.2, 3 and 5 million pixels; colour 0.2, 0.25, 0.64, 1 and 4
 million, widths that are a multiple of 4 and not; levels in one cluster and apart).
 The batched stream, always swept, gives the same bytes; so do float frames of the
 same values; and with FP16 planes and FP64 state."""
@@ -10,7 +10,7 @@ from wema_b200 import cuda as wc
 
 pytestmark = pytest.mark.gpu
 
-LUMA = [(999, 600), (1000, 600), (1095, 1095), (1096, 1096), (640, 578), (642, 579)]
+LUMA = [(999, 600), (1001, 600), (1095, 1095), (1096, 1096), (2236, 2236), (2237, 2236), (3463, 3465), (3465, 3465), (640, 578), (642, 579)]
 COLOR = [(447, 447), (448, 447), (499, 500), (501, 500), (502, 499), (800, 799), (1001, 800), (999, 1000), (1002, 1000),
          (1999, 2000), (2001, 2000), (320, 240), (640, 360)]
 

@@ -823,23 +823,27 @@ cudaError_t launch_dwt_inv_multi(int channels, int out_mode, const InvLevelParam
 
 // ---- one stream's level: by tiles (dwt_tiles.cu) or by sweeps.  A sweep's chain of
 // steps (rows of a segment + 4) is longer than a tile's, so a level that does not
-// fill the GPU several times over is a tile's; with other frames in flight the
-// sweeps' fewer instructions count, which draws the lines for one channel
-// lower.  Level alone, tiles / sweeps, us: forward from RGB24 1280x720 8.3 / 12.8,
-// colour 17.0 / 21.8; 1920x1080 12.4 / 16.3, colour 27.1 / 33.4; 3840x2160 35.8 /
-// 34.9, colour 77 / 92; 320x240 colour 13.6 / 10.8; planes of 640x360 5.0 / 7.0,
-// 1920x1080 9.3 / 10.4, three of them 22.4 / 18.5.  Inverse 1280x720 6.2 / 6.6,
-// 1920x1080 10.0 / 7.6, three planes of 960x540 7.8 / 8.7, of 1280x720 12.6 / 11.3;
-// to RGB 1280x720 16.1 / 11.9, 1366x767 (rows that do not start at words) 14.5 /
-// 16.9, 427x239 11.6 / 8.9.  Frames in flight, before -> with the lines: 1366x767
-// colour 88 -> 68, 1920x1080 colour 111 -> 107, with FP16 planes 1281x719 colour
-// 81 -> 61, 640x480 colour 50 -> 42, 1280x720 64 -> 60; past the lines 1920x1080
-// luma would go 83 -> 86, 3840x2160 colour 364 -> 368.  A level at most two strips
-// wide leaves half of a CTA's warps idle: 33x30000 244 -> 79 in colour.
+// fill the GPU several times over is a tile's; past the lines the sweeps' fewer
+// instructions count, with frames of several sessions in flight above all.  Level
+// alone, tiles / sweeps, us: forward from RGB24 1280x720 8.3 / 12.8, colour 17.0 /
+// 21.8; 1920x1080 12.4 / 16.3, colour 27.1 / 33.4; 3840x2160 35.8 / 34.9, colour 77 /
+// 92; 320x240 colour 13.6 / 10.8; planes of 640x360 5.0 / 7.0, 1920x1080 9.3 / 10.4,
+// three of them 22.4 / 18.5.  Inverse 1280x720 6.2 / 6.6, 1920x1080 10.0 / 7.6, three
+// planes of 960x540 7.8 / 8.7, of 1280x720 12.6 / 11.3; to RGB 1280x720 16.1 / 11.9,
+// 1366x767 (rows that do not start at words) 14.5 / 16.9, 427x239 11.6 / 8.9.
+// Three sessions side by side, us a frame, every level by sweeps / with these lines:
+// 1366x767 48 / 41, colour 75 / 58, 1920x1080 63 / 59, colour 113 / 112, 2560x1440
+// 98 / 94; on the far side of them 3840x2160 luma would go 198 -> 213 and colour
+// 391 -> 407, 1920x1080 with its inverse by tiles 59 -> 60.  One session's frames in
+// flight: 640x480 colour with FP16 planes 49 / 46, 1281x719 81 / 61, 853x479 colour
+// 62 / 50.  (Float frames of one channel go over earlier: 1920x1080, one session,
+// sweeps 110, tiles 118.)  A level at most two strips wide leaves half of a CTA's
+// warps idle: 33x30000 colour 244 / 79.
 static bool fwd_by_tiles(int mode, int channels, const FwdLevelParams& p) {
     const long long px = (long long)p.iw * p.ih;
     if (channels == 3 && mode != kSrcPlanes) return px >= 200000 && (px < 4000000 || dwt_narrow(p.sw));
-    return px < (channels == 1 ? 600000 : 1000000) || dwt_narrow(p.sw);
+    const long long line = channels == 3 ? 1000000 : mode == kSrcRgbU8 ? 5000000 : mode == kSrcPlanes ? 3000000 : 600000;
+    return px < line || dwt_narrow(p.sw);
 }
 static bool inv_by_tiles(int channels, int out_mode, const InvLevelParams& p) {
     const long long px = (long long)p.ow * p.oh;
@@ -885,19 +889,20 @@ cudaError_t launch_dwt_inv(int channels, int out_mode, const InvLevelParams& p0,
 }
 
 // Whether levels from one of sw x sh positions on run in a cluster: at most 6 rows
-// of a strip per warp, in colour 2.  The cluster saves two launches of the host per
-// direction, and is the longer chain on the GPU (levels of 640x480 luma 21 us, by
-// tiles 14).  So it is the faster one where the host bounds the frames in flight:
-// luma 320x240 (1.2 rows) 47 -> 42 us a frame, 640x480 49.8 -> 49.5, with FP16
-// planes 60 -> 49; in colour, whose forward levels bound the frame, 160x120 35 -> 32,
-// 320x240 40 -> 39, but 640x360 (2.8 rows) 42 -> 45, 640x480 44 -> 47.
-constexpr int TAIL_ROWS = 6, TAIL_ROWS_COLOR = 2;
-static bool tail_fits(int sw, int sh, int n, int channels) {
+// of a strip per warp.  The cluster saves two launches of the host per direction and
+// is the longer chain on the GPU (levels of 640x480 21 us, by tiles 14): the faster
+// form where the host bounds the frames.  Three sessions side by side, us a frame, by
+// tiles / in a cluster: luma 320x240 (1.2 rows) 38 / 30; colour 640x360 (2.8) 43.5 /
+// 32, 640x480 (3.8) 43.5 / 32, 853x479 (5.0) 43.6 / 32; 1023x577 (7.6) 43 / 49.  One
+// session's colour frames in flight, which the forward levels bound, pay for it: 640x480
+// 42 / 47, 853x479 48 / 52.
+constexpr int TAIL_ROWS = 6;
+static bool tail_fits(int sw, int sh, int n) {
     const long long rows = (long long)((sw + SW_LANES * SQ - 1) / (SW_LANES * SQ)) * sh;
-    return n >= 2 && n <= 3 && rows <= (channels == 3 ? TAIL_ROWS_COLOR : TAIL_ROWS) * TAIL_CTAS * TAIL_WARPS;
+    return n >= 2 && n <= 3 && rows <= TAIL_ROWS * TAIL_CTAS * TAIL_WARPS;
 }
 cudaError_t launch_dwt_fwd_levels(int channels, const FwdLevelParams* p, int n, cudaStream_t st, int* launches) {
-    if (n > 0 && tail_fits(p[0].sw, p[0].sh, n, channels)) {
+    if (n > 0 && tail_fits(p[0].sw, p[0].sh, n)) {
         LevelTail<FwdLevelParams> t{};
         for (int l = 0; l < n; l++) t.lv[l] = p[l];
         t.count = n;
@@ -913,7 +918,7 @@ cudaError_t launch_dwt_fwd_levels(int channels, const FwdLevelParams* p, int n, 
     return e;
 }
 cudaError_t launch_dwt_inv_levels(int channels, const InvLevelParams* p, int n, cudaStream_t st, int* launches) {
-    if (n > 0 && tail_fits(p[n - 1].sw, p[n - 1].sh, n, channels)) {
+    if (n > 0 && tail_fits(p[n - 1].sw, p[n - 1].sh, n)) {
         LevelTail<InvLevelParams> t{};
         for (int l = 0; l < n; l++) t.lv[l] = p[l];
         t.count = n;
