@@ -560,7 +560,9 @@ WEMA_API void temporal_filter_apply(const TemporalFilter* filt, const TemporalBu
                                     float* delta_phi_filtered, bool bilateral) {
     (void)filt;
     clear_error();
-    if (buf->filled < buf->window_size) {
+    // a buffer whose init was refused has no ring, and no window that could be full
+    if (buf->window_size < 1 || !buf->phase_buffer || buf->filled < buf->window_size) {
+        if (buf->window_size < 1) set_error("window size must be in 1..%d", WEMA_TEMPORAL_WINDOW_MAX);
         memset(delta_phi_filtered, 0, buf->num_positions * sizeof(float));
         return;
     }
