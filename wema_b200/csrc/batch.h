@@ -514,8 +514,8 @@ public:
         // The transforms' form, per group: sweeps where the streams agree in storage
         // type and hold no FP64 state, else tiles.  A kernel of sweeps for every type
         // spills, and the FP64 state's loads need more warps than sweeps have: eight
-        // 1280x720 streams per tick, sweeps -> tiles: state_fp64 391 -> 357 us, a mix
-        // of the variants 422 -> 358, in colour 837 -> 620.
+        // 1280x720 streams per tick, sweeps -> tiles: state_fp64 391 -> 314 us, a mix
+        // of the variants 422 -> 341, in colour 837 -> 579.
         int fform[MAXG], iform[MAXG];
         for (int g = 0; g < G; g++) {
             bool some16 = false, all16 = true, wide = false;

@@ -836,7 +836,7 @@ cudaError_t launch_dwt_inv_multi(int channels, int out_mode, const InvLevelParam
 // 98 / 94; on the far side of them 3840x2160 luma would go 198 -> 213 and colour
 // 391 -> 407, 1920x1080 with its inverse by tiles 59 -> 60.  One session's frames in
 // flight: 640x480 colour with FP16 planes 49 / 46, 1281x719 81 / 61, 853x479 colour
-// 62 / 50.  (Float frames of one channel go over earlier: 1920x1080, one session,
+// 58 / 52.  (Float frames of one channel go over earlier: 1920x1080, one session,
 // sweeps 110, tiles 118.)  A level at most two strips wide leaves half of a CTA's
 // warps idle: 33x30000 colour 244 / 79.
 static bool fwd_by_tiles(int mode, int channels, const FwdLevelParams& p) {

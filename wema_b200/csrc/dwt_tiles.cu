@@ -1,6 +1,6 @@
-// dwt_tiles.cu - the DWT levels by tiles: where the sweeps of dwt.cu are the slower
+// dwt_tiles.cu - the DWT levels by tiles, where the sweeps of dwt.cu are the slower
 // form: batched launches that hold FP64 filter state or differ in storage type
-// (batch.h has the rule), and small levels of one stream (dwt.cu has it).
+// (batch.h has the rule), and the smaller levels of one stream (dwt.cu has it).
 //
 // A CTA owns a tile of TP x TP subband pairs (TP = 27) and stages a 64 x 64
 // sample region - the tile's 54 samples plus a 4-sample halo before and a
